@@ -33,6 +33,8 @@ SOURCES = [
     "gsls_noalloc.cu",
     "gsls_ns.cu",
     "gsls_bicgs.cu",
+    "gsls_part.cu",
+    "gsls_wcg.cu",
 ]
 
 

@@ -86,6 +86,22 @@ struct KrylovScalars {
   double pad1[3];
 };
 
+// device scalar buffer: KrylovScalars and, at kScalRed, the counter, error
+// word and partials of a grid sum (GridRedBuf); the first kScalHost bytes
+// (scalars, counter, error word) are what the host reads back
+constexpr size_t kScalRed = 128, kScalHost = 144;
+constexpr size_t kScalBytes = kScalRed + 16 + 2 * 256 * 16;
+static_assert(sizeof(KrylovScalars) <= kScalRed, "scalar block");
+
+// Row partition of the persistent kernels (gsls_part.cuh)
+struct RowPart {
+  bool built = false, ok = false;
+  int nblk = 0, L = 1, winMax = 0, nslMax = 0, stMax = 0;
+  long long slots = 0, steps = 0;
+  DevBuf buf;           // the tables of PartArgs at their offsets
+  size_t off[8] = {};
+};
+
 // Face (BC) description, FSILS_faceType.
 struct Face {
   bool foC = false, coupledFlag = false, sharedFlag = false, incFlag = true;
@@ -142,10 +158,15 @@ struct Workspace {
   int sell_D = 0, sell_nS = 0, sell_vkey = 0;
   long long sell_steps = 0;
   DevBuf sell_off, sell_row, sell_col, sell_pos, sell_val;
+  // row partition; stream and vectors of the windowed CG (gsls_wcg.cu)
+  RowPart part;
+  DevBuf wcg_stream, wcg_vec;
+  unsigned long long wcg_serial = 0;  // preconditioning whose matrix the stream holds
+  const void *wcg_val = nullptr;      // (and the array it was packed from)
+  int wcg_key = 0;                    // block size and value type of the stream
   DevBuf partials;    // double[grid * 64]
   DevBuf ticket;      // unsigned[8]
-  DevBuf scal;        // KrylovScalars
-  DevBuf cgbar;       // grid barrier of the persistent CG
+  DevBuf scal;        // KrylovScalars; then GridRedBuf
   DevBuf vec[6];      // Krylov work vectors (X, P, KP, R32...)
   DevBuf W;           // diag preconditioner (double dof x nNo)
   DevBuf W2;          // RCS second scaling
@@ -363,6 +384,11 @@ int cpl_prepare(gsls_lhs *lhs, int dof, const double *dW, int prec);
 // vectors with vdof values per node; skipped when *done is set
 template <class XT>
 void launch_addbcmul(gsls_lhs *lhs, int op, int vdof, const XT *X, XT *Y, const int *done);
+// CG on the preconditioned system as one cooperative launch (gsls_wcg.cu);
+// R in: rhs, out: W X.  keep: Val is what the last preconditioning on this
+// lhs left.  *ran false: the partition's windows do not fit, nothing done.
+int wcg_run(gsls_lhs *lhs, gsls_sub_ls *ls, int D, bool mixed, const void *Val, double *R,
+            const double *W, bool keep, bool *ran);
 // BiCGStab on the preconditioned system (gsls_bicgs.cu)
 int bicgs_run(gsls_lhs *lhs, gsls_sub_ls *ls, int D, bool mixed, const void *Val, double *R,
               const double *W);

@@ -121,7 +121,7 @@ int lhs_prepare_ws(gsls_lhs *lhs, int dof) {
     GSLS_TRY(ws.ticket.alloc(sizeof(unsigned) * 256));
     GSLS_CUDA(cudaMemsetAsync(ws.ticket.p, 0, sizeof(unsigned) * 256, lhs->stream));
   }
-  GSLS_TRY(ws.scal.alloc(sizeof(KrylovScalars)));
+  GSLS_TRY(ws.scal.alloc(kScalBytes));
   for (int k = 0; k < 6; k++) GSLS_TRY(ws.vec[k].alloc(sizeof(double) * nv));
   GSLS_TRY(ws.W.alloc(sizeof(double) * nv));
   GSLS_TRY(ws.W2.alloc(sizeof(double) * nv));
@@ -132,8 +132,8 @@ int lhs_prepare_ws(gsls_lhs *lhs, int dof) {
   }
   GSLS_TRY(ws.mask.alloc(sizeof(double) * nv));
   if (!ws.h_scal) {
-    GSLS_CUDA(cudaMallocHost(&ws.h_scal, sizeof(KrylovScalars)));
-    memset(ws.h_scal, 0, sizeof(KrylovScalars));
+    GSLS_CUDA(cudaMallocHost(&ws.h_scal, kScalHost));
+    memset(ws.h_scal, 0, kScalHost);
   }
   return GSLS_OK;
 }

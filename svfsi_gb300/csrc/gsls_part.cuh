@@ -1,0 +1,120 @@
+// Row partition of the matrix over the thread blocks of a persistent Krylov
+// kernel (one block per SM), with the matrix in a per-warp stream layout.
+//
+// Block b owns a compact set of rows.  Every vector entry that its rows
+// multiply is either its own or in its halo list, so a block that keeps both
+// in shared memory (its window) reads no vector entry from L2 inside the
+// product: one coalesced pass over the halo replaces ~15 scattered gathers
+// per row.  Columns become 16-bit window indices.
+//
+// Order: a block's rows, sorted by decreasing length, fill slices of
+// RW = 32/L rows; lane g*L + l of a slice's warp takes the blocks l, l+L, ...
+// of row g.  Vectors of the kernel live in this slot order (slot = slice*RW +
+// g over all blocks; empty slots hold zeros).  Slice s of a block belongs to
+// warp s % kPartWarps, and a warp's steps are those of its slices one after another.
+#pragma once
+
+#include "gsls_internal.cuh"
+
+namespace gsls {
+
+// Warps per block: FP64 instructions issue at one per ~64 cycles and
+// scheduler whatever the number of warps, and each warp pays for its own
+// share of every reduction; in FP32, 16 warps of 128 registers spill and were
+// 12 % slower on the beam than 8 (122 against 107 ms a step).
+constexpr int kPartWarps = 8;
+constexpr int kPartThreads = 32 * kPartWarps;
+constexpr int kPartMaxBlocks = 256;
+
+struct PartArgs {
+  const int *wbase;   // first step of each (block, warp), nblk * kPartWarps + 1
+  const int *sbase;   // first slice of each block, nblk + 1
+  const int *slen;    // steps of each slice (>= 1)
+  const int *hoff;    // halo offsets, nblk + 1
+  const int *halo;    // halo entries: slots of other blocks
+  const int *slotRow; // row of each slot or -1
+  const int *src;     // CSR block of each (step, lane) or -1
+  const unsigned short *lcol;  // window index of each (step, lane)
+  int nblk, L;
+  int winMax, nslMax, stMax;  // largest window, slices and steps of a warp
+  long long nslots, nsteps;
+};
+
+// Partition of the lhs over at most num_sms() blocks; built on the host once
+// per lhs.  ok is false when a window has more than 65,535 entries.
+int part_setup(gsls_lhs *lhs);
+PartArgs part_args(const RowPart &p);
+
+// A node's D values in global memory, read and written through L2; stride VD
+// (3-vectors are padded to 4 values: whole 16-byte accesses)
+template <int D, class XT>
+struct NodeL2 {
+  static constexpr int VD = D == 3 ? 4 : D;
+  static __device__ __forceinline__ void ld(const XT *p, XT o[D]) {
+    if constexpr (sizeof(XT) == 4) {
+      if constexpr (D == 1) {
+        o[0] = __ldcg(p);
+      } else if constexpr (D == 2) {
+        const float2 v = __ldcg(reinterpret_cast<const float2 *>(p));
+        o[0] = v.x;
+        o[1] = v.y;
+      } else {
+        const float4 v = __ldcg(reinterpret_cast<const float4 *>(p));
+        o[0] = v.x;
+        o[1] = v.y;
+        o[2] = v.z;
+        if constexpr (D == 4) o[3] = v.w;
+      }
+    } else {
+      if constexpr (D == 1) {
+        o[0] = __ldcg(p);
+      } else {
+        const double2 v = __ldcg(reinterpret_cast<const double2 *>(p));
+        o[0] = v.x;
+        o[1] = v.y;
+        if constexpr (D > 2) {
+          const double2 u = __ldcg(reinterpret_cast<const double2 *>(p) + 1);
+          o[2] = u.x;
+          if constexpr (D == 4) o[3] = u.y;
+        }
+      }
+    }
+  }
+  static __device__ __forceinline__ void st(XT *p, const XT o[D]) {
+    if constexpr (sizeof(XT) == 4) {
+      if constexpr (D == 1)
+        __stcg(p, o[0]);
+      else if constexpr (D == 2)
+        __stcg(reinterpret_cast<float2 *>(p), make_float2(o[0], o[1]));
+      else
+        __stcg(reinterpret_cast<float4 *>(p), make_float4(o[0], o[1], o[2], D == 4 ? o[D - 1] : 0.f));
+    } else {
+      if constexpr (D == 1) {
+        __stcg(p, o[0]);
+      } else {
+        __stcg(reinterpret_cast<double2 *>(p), make_double2(o[0], o[1]));
+        if constexpr (D > 2)
+          __stcg(reinterpret_cast<double2 *>(p) + 1, make_double2(o[2], D == 4 ? o[D - 1] : 0.0));
+      }
+    }
+  }
+};
+
+// use(k, load(k)) for the nodes k of this thread, B loads in flight
+template <int D, class XT>
+constexpr int kB = sizeof(XT) == 4 ? 6 : D > 2 ? 3 : 5;
+template <int B, int D, class XT, class Ld, class Use>
+__device__ __forceinline__ void for_nodes(int n, const Ld &load, const Use &use) {
+#pragma unroll 1
+  for (int k0 = threadIdx.x; k0 < n; k0 += B * kPartThreads) {
+    XT v[B][D];
+#pragma unroll
+    for (int u = 0; u < B; u++)
+      if (k0 + u * kPartThreads < n) load(k0 + u * kPartThreads, v[u]);
+#pragma unroll
+    for (int u = 0; u < B; u++)
+      if (k0 + u * kPartThreads < n) use(k0 + u * kPartThreads, v[u]);
+  }
+}
+
+}  // namespace gsls
