@@ -505,7 +505,7 @@ def run_gsls(args):
             B = p.nnz * (7 * s + 4) + 4 * p.nNo + 16 * p.nNo * s
             it_s = (tot_ms / max(cnt, 1)) / 1e3
             ach = B / it_s / 1e9 if cnt else None
-            return {"kernel": f"k_schur_persistent<{t},{t}> (CGRAD_SCHUR: every CG iteration "
+            return {"kernel": f"k_wschur<{t},{t}> (CGRAD_SCHUR: every CG iteration "
                               "of one call in one cooperative launch, 3 grid barriers per "
                               "iteration)",
                     "bound": "l2", "achieved": ach, "peak": l2rate, "unit": "GB/s",

@@ -35,6 +35,7 @@ SOURCES = [
     "gsls_bicgs.cu",
     "gsls_part.cu",
     "gsls_wcg.cu",
+    "gsls_wschur.cu",
 ]
 
 

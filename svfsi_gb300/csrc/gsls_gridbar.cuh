@@ -27,48 +27,6 @@ __device__ __forceinline__ unsigned ld_acquire_gpu(const unsigned *p) {
   asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
-__device__ __forceinline__ bool grid_bar(GridBar *b, unsigned nblk, unsigned &epoch,
-                                         unsigned limit) {
-  __shared__ int s_ok;
-  __syncthreads();
-  epoch += 1;
-  if (threadIdx.x == 0) {
-    int ok = 1;
-    const unsigned target = epoch * nblk;
-    asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(&b->count), "r"(1u) : "memory");
-    unsigned it = 0;
-    while (ld_acquire_gpu(&b->count) < target) {
-      ++it;
-      if ((it & 31u) == 0u && *(volatile int *)&b->err) {
-        ok = 0;
-        break;
-      }
-      if (it > limit) {
-        atomicExch(&b->err, 1);
-        ok = 0;
-        break;
-      }
-      if (it > 64u) __nanosleep(20);
-    }
-    s_ok = ok;
-  }
-  __syncthreads();
-  return s_ok != 0;
-}
-
-// sum of nblk block partials in block order, broadcast to the block
-__device__ __forceinline__ double sum_partials(const double *part, unsigned nblk, double *sh) {
-  double v = 0.0;
-  for (unsigned k = threadIdx.x; k < nblk; k += blockDim.x) v += __ldcg(part + k);
-  v = block_sum(v, sh);
-  __shared__ double s_tot;
-  if (threadIdx.x == 0) s_tot = v;
-  __syncthreads();
-  const double r = s_tot;
-  __syncthreads();
-  return r;
-}
-
 // Grid-wide sum that is also a grid barrier, split into arrive and wait so
 // that a block can work between the two.  Thread 0 writes the block's partial
 // and then adds one to a counter (release); lane 0 of warp 0 polls the counter

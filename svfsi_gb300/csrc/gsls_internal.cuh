@@ -96,10 +96,10 @@ static_assert(sizeof(KrylovScalars) <= kScalRed, "scalar block");
 // Row partition of the persistent kernels (gsls_part.cuh)
 struct RowPart {
   bool built = false, ok = false;
-  int nblk = 0, L = 1, winMax = 0, nslMax = 0, stMax = 0;
-  long long slots = 0, steps = 0;
+  int nblk = 0, L = 1, winMax = 0, nslMax = 0, stMax = 0, grpMax = 0, nS = 0;
+  long long slots = 0, steps = 0, steps8 = 0;
   DevBuf buf;           // the tables of PartArgs at their offsets
-  size_t off[8] = {};
+  size_t off[10] = {};
 };
 
 // Face (BC) description, FSILS_faceType.
@@ -176,6 +176,7 @@ struct Workspace {
   DevBuf io;          // host<->device staging for gsls_solve
   DevBuf io2;
   DevBuf ns_vec;      // NS solver vectors (Rm, Rc, U, P, MU, MP, Schur CG)
+  DevBuf ns_stream;   // streams and published vectors of the Schur CG (gsls_wschur.cu)
   DevBuf ns_mat;      // NS solver blocks (mK, mG, mD, mL, Gt)
   DevBuf rcs;         // RCS scaling state (W1, Wr, Wc, control words)
   DevBuf cpl_glob, cpl_valM;  // coupled faces of the current solve

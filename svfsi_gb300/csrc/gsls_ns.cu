@@ -13,8 +13,8 @@
 //    transpose map, no atomics) and only the final pass rewrites Val;
 //  * NSSOLVER's DEPART split (mK 3x3, mG 3x1, mD 1x3, mL, Gt = -mG^T) is one
 //    kernel; the rectangular products SPARMULVS/SV/SS use 4 lanes per block
-//    row; the Schur CG runs device-resident with the host polling a scalar
-//    block every 8 iterations; the <= 20 x 20 least-squares system of each
+//    row; each Schur CG is one cooperative launch (gsls_wschur.cu; with
+//    coupled faces a batch of kernels per 8 iterations); the <= 20 x 20 least-squares system of each
 //    outer iteration is solved on the host (GE).
 // Vectors are in the Krylov type XT (FP32 in mixed mode), scalars in FP64.
 #include <algorithm>
@@ -24,8 +24,9 @@
 #include <vector>
 
 #include "gsls_internal.cuh"
-#include "gsls_gridbar.cuh"
+#include "gsls_part.cuh"
 #include "gsls_spmv.cuh"
+#include "gsls_wschur.cuh"
 
 namespace gsls {
 
@@ -303,11 +304,10 @@ __global__ void __launch_bounds__(kNT) k_ns_split(int nNo, const double *__restr
   }
 }
 
-// DEPART (NSSOLVER.f:237-305) for nsd = 3.  Also writes the Schur operands
-// packed four to a block for the persistent CG: A1 = (mG, 0), A2 = (Gt, mL).
+// DEPART (NSSOLVER.f:237-305) for nsd = 3
 template <class VT>
 __global__ void k_depart(int nnz, const VT *__restrict__ Val, const int *__restrict__ tpos, VT *mK,
-                         VT *mG, VT *mD, VT *mL, VT *Gt, VT *A1, VT *A2) {
+                         VT *mG, VT *mD, VT *mL, VT *Gt) {
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < nnz; j += gridDim.x * blockDim.x) {
     const VT *t = Val + (size_t)j * 16;
     VT *k = mK + (size_t)j * 9;
@@ -322,46 +322,10 @@ __global__ void k_depart(int nnz, const VT *__restrict__ Val, const int *__restr
       mG[(size_t)j * 3 + m] = g;
       mD[(size_t)j * 3 + m] = t[12 + m];
       Gt[(size_t)l * 3 + m] = -g;
-      A1[(size_t)j * 4 + m] = g;
-      A2[(size_t)l * 4 + m] = -g;
     }
-    A1[(size_t)j * 4 + 3] = VT(0);
     mL[j] = t[15];
-    A2[(size_t)j * 4 + 3] = t[15];
   }
 }
-
-// 16-byte (FP32) / 2 x 16-byte (FP64) vector access to 4 packed values
-template <class T> struct V4;
-template <> struct V4<float> {
-  static __device__ __forceinline__ void ldg(const float *p, float o[4]) {
-    const float4 v = __ldg(reinterpret_cast<const float4 *>(p));
-    o[0] = v.x; o[1] = v.y; o[2] = v.z; o[3] = v.w;
-  }
-  static __device__ __forceinline__ void ldcg(const float *p, float o[4]) {
-    const float4 v = __ldcg(reinterpret_cast<const float4 *>(p));
-    o[0] = v.x; o[1] = v.y; o[2] = v.z; o[3] = v.w;
-  }
-  static __device__ __forceinline__ void stcg(float *p, float a, float b, float c, float d) {
-    __stcg(reinterpret_cast<float4 *>(p), make_float4(a, b, c, d));
-  }
-};
-template <> struct V4<double> {
-  static __device__ __forceinline__ void ldg(const double *p, double o[4]) {
-    const double2 a = __ldg(reinterpret_cast<const double2 *>(p));
-    const double2 b = __ldg(reinterpret_cast<const double2 *>(p) + 1);
-    o[0] = a.x; o[1] = a.y; o[2] = b.x; o[3] = b.y;
-  }
-  static __device__ __forceinline__ void ldcg(const double *p, double o[4]) {
-    const double2 a = __ldcg(reinterpret_cast<const double2 *>(p));
-    const double2 b = __ldcg(reinterpret_cast<const double2 *>(p) + 1);
-    o[0] = a.x; o[1] = a.y; o[2] = b.x; o[3] = b.y;
-  }
-  static __device__ __forceinline__ void stcg(double *p, double a, double b, double c, double d) {
-    __stcg(reinterpret_cast<double2 *>(p), make_double2(a, b));
-    __stcg(reinterpret_cast<double2 *>(p) + 1, make_double2(c, d));
-  }
-};
 
 // 4 lanes per block row, 8 rows per warp; lane q takes blocks rs+q, rs+q+4, ...
 constexpr int kRL = 4;
@@ -462,12 +426,6 @@ __global__ void __launch_bounds__(kNT) k_ns_ss_vs(int nNo, const int *__restrict
     }
   }
 }
-
-// Schur CG scalar block (CGRAD_SCHUR, CGRAD.f:51-123)
-struct SchurScal {
-  double err, errO, eps, dot, iNorm2;
-  int done, suc, itr, mItr;
-};
 
 // X = 0, Rs = Ps = P (in), |P|^2 -> err; decides the first stop test
 template <class XT>
@@ -733,274 +691,12 @@ static bool ge_solve(int nV, int N, const std::vector<double> &A, std::vector<do
   return true;
 }
 
-// ---------------------------------------------------------------------------
-// Persistent Schur CG: every iteration of CGRAD_SCHUR in one cooperative
-// launch.  Phases are separated by a grid barrier (generation counter; each
-// wait is bounded and sets an error word when it gives up, after which
-// every block returns).  Data written by other blocks is read through L2
-// (__ldcg); the matrix blocks are read-only.  Reductions: one FP64 partial
-// per block, summed in block order by every block (identical result in all
-// blocks, reproducible for a fixed grid).
-template <class VT, class XT>
-struct SchurArgs {
-  int nNo;
-  const int *rowPtr, *colPtr;
-  const VT *A1, *A2;              // (mG, 0) and (Gt, mL) per CSR block
-  XT *X, *Pa, *Pb, *R, *SP, *GP;  // Pa holds the initial direction; GP 4 per node
-  double *part;                   // 2 * gridDim.x
-  GridBar *bar;
-  SchurScal *sc;
-  int K;                          // rows per 4-lane group (row slots)
-  int zz;                         // reverse the row-slot order on odd iterations
-  unsigned spin;                  // poll limit of the grid barrier
-};
-
-constexpr int kPT = 1024;
-constexpr int kPQ = kPT / kRL;  // 4-lane groups per block
-
-// Row slots of a block: slot (k, g) is row blockIdx.x*kPQ + g + k*gridDim.x*kPQ.
-// The K segments of a block are contiguous in the CSR; their column
-// indices and row ranges are staged in shared memory once per launch:
-//   srp[k*kPQ + g] = (first, end) of the row in scol, sdel[k] = global - local
-__device__ __forceinline__ void schur_stage(const int *__restrict__ rowPtr,
-                                            const int *__restrict__ colPtr, int nNo, int K,
-                                            int2 *srp, int *sdel, int *scol) {
-  const int nq = gridDim.x * kPQ;
-  int off = 0;
-  for (int k = 0; k < K; k++) {
-    const int base = blockIdx.x * kPQ + k * nq;
-    if (base >= nNo) {
-      if (threadIdx.x < kPQ) srp[k * kPQ + threadIdx.x] = make_int2(0, 0);
-      if (threadIdx.x == 0) sdel[k] = 0;
-      continue;
-    }
-    const int hi = min(base + kPQ, nNo);
-    const int s0 = __ldg(rowPtr + base), s1 = __ldg(rowPtr + hi);
-    for (int j = threadIdx.x; j < s1 - s0; j += blockDim.x) scol[off + j] = __ldg(colPtr + s0 + j);
-    if (threadIdx.x < kPQ) {
-      const int i = base + threadIdx.x;
-      srp[k * kPQ + threadIdx.x] =
-          (i < nNo) ? make_int2(__ldg(rowPtr + i) - s0 + off, __ldg(rowPtr + i + 1) - s0 + off)
-                    : make_int2(0, 0);
-    }
-    if (threadIdx.x == 0) sdel[k] = s0 - off;
-    off += s1 - s0;
-  }
-  __syncthreads();
-}
-
-// Iteration k of CGRAD_SCHUR (CGRAD.f:86-110), three phases:
-//  1. P_k = (err/errO) (P_{k-1} + (errO/err) R) formed on the fly from the
-//     previous direction (the reference's two OMPSUMS/OMPMULS steps; P_1 = R
-//     exactly with errO/err = 0, err/errO = 1) and GP = mG P_k; the owner of
-//     row i stores P_k(i) in the other buffer;
-//  2. SP = mL P_k - Gt GP and the block partials of P_k.SP;
-//  3. alpha = errO/dot, X += alpha P_k, R -= alpha SP and the partials of |R|^2.
-// With zz set, odd iterations visit the row slots last to first, so the
-// operator blocks read at the end of one pass are the first read by the
-// next and are still in L2 when the operator does not fit there whole.
-template <class VT, class XT>
-__global__ void __launch_bounds__(kPT, 1) k_schur_persistent(SchurArgs<VT, XT> A) {
-  using AT = typename AccOf<VT>::T;
-  constexpr int kPU = sizeof(AT) == 4 ? 4 : 2;  // blocks per lane issued together
-  extern __shared__ int4 smem_raw[];
-  int2 *srp = reinterpret_cast<int2 *>(smem_raw);
-  int *sdel = reinterpret_cast<int *>(srp + A.K * kPQ);
-  int *scol = sdel + ((A.K + 3) & ~3);
-  __shared__ double sh[32];
-  const unsigned nblk = gridDim.x;
-  const int nNo = A.nNo, K = A.K;
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  const int nthr = gridDim.x * blockDim.x;
-  const int q = t & (kRL - 1), g = threadIdx.x / kRL;
-  const int nq = gridDim.x * kPQ;
-  double err = A.sc->err;
-  const double eps = A.sc->eps;
-  const int mItr = A.sc->mItr;
-  int done = A.sc->done, suc = A.sc->suc, itr = 0;
-  double errO = A.sc->errO;
-  XT c1 = XT(0), c2 = XT(1);
-  XT *Pold = A.Pa, *Pnew = A.Pb;
-  bool ok = true;
-  unsigned epoch = 0;
-  schur_stage(A.rowPtr, A.colPtr, nNo, K, srp, sdel, scol);
-  while (!done) {
-    const bool rev = A.zz && (itr & 1);
-    // phase 1: P_k on the fly, GP = mG P_k
-    for (int kk = 0; kk < K; kk++) {
-      const int k = rev ? K - 1 - kk : kk;
-      const int i = blockIdx.x * kPQ + g + k * nq;
-      if ((i & ~7) >= nNo) continue;  // warp-uniform: a warp covers 8 consecutive rows
-      const int2 rr = srp[k * kPQ + g];
-      const int dl = sdel[k];
-      // the owner's own entry of P_k, loaded before the gathers
-      XT pown = XT(0);
-      if (q == 0 && i < nNo) pown = XT(c2 * (__ldcg(Pold + i) + c1 * __ldcg(A.R + i)));
-      AT a0 = AT(0), a1 = AT(0), a2 = AT(0);
-      for (int j0 = rr.x + q; j0 < rr.y; j0 += kPU * kRL) {
-        AT pv[kPU], gv[kPU][3];
-#pragma unroll
-        for (int u = 0; u < kPU; u++) {
-          const int jl = j0 + u * kRL;
-          if (jl < rr.y) {
-            const int col = scol[jl];
-            const size_t j = (size_t)(jl + dl);
-            pv[u] = AT(c2 * (__ldcg(Pold + col) + c1 * __ldcg(A.R + col)));
-            VT a4[4];
-            V4<VT>::ldg(A.A1 + j * 4, a4);
-#pragma unroll
-            for (int m = 0; m < 3; m++) gv[u][m] = AT(a4[m]);
-          } else {
-            pv[u] = AT(0);
-#pragma unroll
-            for (int m = 0; m < 3; m++) gv[u][m] = AT(0);
-          }
-        }
-#pragma unroll
-        for (int u = 0; u < kPU; u++) {
-          a0 = fma(gv[u][0], pv[u], a0);
-          a1 = fma(gv[u][1], pv[u], a1);
-          a2 = fma(gv[u][2], pv[u], a2);
-        }
-      }
-      a0 = quad_sum(a0);
-      a1 = quad_sum(a1);
-      a2 = quad_sum(a2);
-      if (q == 0 && i < nNo) {
-        V4<XT>::stcg(A.GP + (size_t)i * 4, XT(a0), XT(a1), XT(a2), XT(0));
-        __stcg(Pnew + i, pown);
-      }
-    }
-    if (!(ok = grid_bar(A.bar, nblk, epoch, A.spin))) break;
-    // phase 2: SP = mL P - Gt GP; dot = P.SP
-    AT dloc = AT(0);
-    for (int kk = 0; kk < K; kk++) {
-      const int k = rev ? K - 1 - kk : kk;
-      const int i = blockIdx.x * kPQ + g + k * nq;
-      if ((i & ~7) >= nNo) continue;
-      const int2 rr = srp[k * kPQ + g];
-      const int dl = sdel[k];
-      const AT pown = (q == 0 && i < nNo) ? AT(__ldcg(Pnew + i)) : AT(0);
-      AT sl = AT(0), sd = AT(0);
-      for (int j0 = rr.x + q; j0 < rr.y; j0 += kPU * kRL) {
-        AT lv[kPU], pv[kPU], gt[kPU][3], gp[kPU][3];
-#pragma unroll
-        for (int u = 0; u < kPU; u++) {
-          const int jl = j0 + u * kRL;
-          if (jl < rr.y) {
-            const int col = scol[jl];
-            const size_t j = (size_t)(jl + dl);
-            VT a4[4];
-            V4<VT>::ldg(A.A2 + j * 4, a4);
-            XT g4[4];
-            V4<XT>::ldcg(A.GP + (size_t)col * 4, g4);
-            lv[u] = AT(a4[3]);
-            pv[u] = AT(__ldcg(Pnew + col));
-#pragma unroll
-            for (int m = 0; m < 3; m++) {
-              gt[u][m] = AT(a4[m]);
-              gp[u][m] = AT(g4[m]);
-            }
-          } else {
-            lv[u] = pv[u] = AT(0);
-#pragma unroll
-            for (int m = 0; m < 3; m++) gt[u][m] = gp[u][m] = AT(0);
-          }
-        }
-#pragma unroll
-        for (int u = 0; u < kPU; u++) {
-          sl = fma(lv[u], pv[u], sl);
-#pragma unroll
-          for (int m = 0; m < 3; m++) sd = fma(gt[u][m], gp[u][m], sd);
-        }
-      }
-      sl = quad_sum(sl);
-      sd = quad_sum(sd);
-      if (q == 0 && i < nNo) {
-        const XT v = XT(sl + AT(-1) * sd);
-        __stcg(A.SP + i, v);
-        dloc = fma(pown, AT(v), dloc);
-      }
-    }
-    {
-      const double bs = block_sum(double(dloc), sh);
-      if (threadIdx.x == 0) __stcg(A.part + blockIdx.x, bs);
-    }
-    if (!(ok = grid_bar(A.bar, nblk, epoch, A.spin))) break;
-    // phase 3: X, R and |R|^2
-    const double dot = sum_partials(A.part, nblk, sh);
-    errO = err;
-    const double alpha = errO / dot;
-    const XT al = XT(alpha), mal = XT(-alpha);
-    double eloc = 0.0;
-    for (int k = t; k < nNo; k += nthr) {
-      __stcg(A.X + k, XT(__ldcg(A.X + k) + al * __ldcg(Pnew + k)));
-      const XT r = XT(__ldcg(A.R + k) + mal * __ldcg(A.SP + k));
-      __stcg(A.R + k, r);
-      eloc += double(r) * double(r);
-    }
-    {
-      const double bs = block_sum(eloc, sh);
-      if (threadIdx.x == 0) __stcg(A.part + nblk + blockIdx.x, bs);
-    }
-    if (!(ok = grid_bar(A.bar, nblk, epoch, A.spin))) break;
-    double e = sqrt(sum_partials(A.part + nblk, nblk, sh));
-    e = e * e;
-    err = e;
-    itr++;
-    c1 = XT(errO / err);
-    c2 = XT(err / errO);
-    XT *tmp = Pold;
-    Pold = Pnew;
-    Pnew = tmp;
-    if (!isfinite(err)) {
-      done = 3;
-    } else if (itr >= mItr) {
-      done = 2;  // no stop test after the last iteration
-    } else if (err < eps) {
-      suc = 1;
-      done = 1;
-    }
-  }
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    SchurScal *sc = A.sc;
-    sc->err = err;
-    sc->errO = errO;
-    sc->itr = itr;
-    sc->suc = suc;
-    sc->done = ok ? done : 4;
-  }
-}
-
-// Launch geometry of the persistent Schur CG: one block per SM, K row slots
-// per 4-lane group, shared memory for the staged rows of the largest block
-// (0 when it does not fit: the caller then uses the per-kernel path).
-static size_t schur_geometry(const gsls_lhs *lhs, int nblk, int *K_out) {
-  const int nNo = lhs->nNo, nq = nblk * kPQ;
-  const int K = (nNo + nq - 1) / nq;
-  const std::vector<int> &rp = lhs->h_rowPtr;
-  long long mx = 0;
-  for (int b = 0; b < nblk; b++) {
-    long long tot = 0;
-    for (int k = 0; k < K; k++) {
-      const int base = b * kPQ + k * nq;
-      if (base >= nNo) break;
-      const int hi = std::min(base + kPQ, nNo);
-      tot += rp[hi] - rp[base];
-    }
-    mx = std::max(mx, tot);
-  }
-  *K_out = K;
-  const size_t bytes = (size_t)K * kPQ * sizeof(int2) + (size_t)((K + 3) & ~3) * sizeof(int) +
-                       (size_t)mx * sizeof(int);
-  return bytes <= 200 * 1024 ? bytes : 0;
-}
-
-// CGRAD_SCHUR on P (in: right-hand side, out: solution)
+// CGRAD_SCHUR on P (in: right-hand side, out: solution).  windowed: the
+// operands are laid out for the one-launch kernel (gsls_wschur.cu).
 template <class VT, class XT>
 static int schur_cg(gsls_lhs *lhs, gsls_sub_ls *ls, const VT *mG, const VT *Gt, const VT *mL,
-                    const VT *A1, const VT *A2, XT *P, XT *Rs, XT *Ps, XT *Pb, XT *SP, XT *GP,
-                    XT *GP4, SchurScal *sc, SchurScal *h_sc, GridBar *db) {
+                    XT *P, XT *Rs, XT *Ps, XT *SP, XT *GP, SchurScal *sc, SchurScal *h_sc,
+                    bool windowed) {
   cudaStream_t st = lhs->stream;
   const int nNo = lhs->nNo, G = lhs->grid;
   double *part = lhs->ws.partials.as<double>();
@@ -1008,66 +704,19 @@ static int schur_cg(gsls_lhs *lhs, gsls_sub_ls *ls, const VT *mG, const VT *Gt, 
   const int *rp = lhs->d_rowPtr.as<int>(), *cp = lhs->d_colPtr.as<int>();
   auto t0 = std::chrono::steady_clock::now();
   ls->suc = 0;
-  k_schur_init<XT><<<G, kNT, 0, st>>>(nNo, P, Rs, Ps, part, tk, sc, ls->absTol, ls->relTol, ls->mItr);
-  GSLS_CHECK_LAUNCH();
-  static const bool kernels = [] {
-    const char *e = getenv("GSLS_SCHUR");
-    return e && strcmp(e, "kernels") == 0;
-  }();
-  // the coupled-face PRE term needs a global dot between the two Schur
-  // products: the per-kernel path carries it
-  bool use_kernels = kernels || lhs->ws.cpl_on;
-  if (!use_kernels) {
-    // persistent cooperative kernel: one block per SM
-    const int nblk = num_sms();
-    int K = 0;
-    const size_t smem = schur_geometry(lhs, nblk, &K);
-    int nb = 0;
-    if (smem) {
-      GSLS_CUDA(cudaFuncSetAttribute(k_schur_persistent<VT, XT>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      GSLS_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_schur_persistent<VT, XT>, kPT,
-                                                              smem));
+  if (windowed) {
+    GSLS_TRY((wschur_run<VT, XT>(lhs, ls, P, h_sc)));
+    if (h_sc->done == 4) {
+      set_error("NS: grid barrier of the Schur-complement CG timed out");
+      return GSLS_ERR_CUDA;
     }
-    if (nb < 1) {
-      use_kernels = true;  // rows of a block do not fit in shared memory
-    } else {
-      GSLS_TRY(lhs->ws.partials.alloc(sizeof(double) * ((size_t)2 * nblk + 64) + 64));
-      GSLS_CUDA(cudaMemsetAsync(db, 0, sizeof(GridBar), st));
-      SchurArgs<VT, XT> a{nNo, rp, cp, A1, A2, P, Ps, Pb, Rs, SP, GP4,
-                          lhs->ws.partials.as<double>(), db, sc, K, zigzag_on(),
-                          wait_limit()};
-      void *args[] = {&a};
-      const bool prof = prof_on();
-      cudaEvent_t pe0 = nullptr, pe1 = nullptr;
-      if (prof) {
-        GSLS_CUDA(cudaEventCreate(&pe0));
-        GSLS_CUDA(cudaEventCreate(&pe1));
-        GSLS_CUDA(cudaEventRecord(pe0, st));
-      }
-      GSLS_CUDA(cudaLaunchCooperativeKernel((const void *)k_schur_persistent<VT, XT>, dim3(nblk),
-                                            dim3(kPT), args, smem, st));
-      GSLS_CHECK_LAUNCH();
-      if (prof) GSLS_CUDA(cudaEventRecord(pe1, st));
-      GSLS_CUDA(cudaMemcpyAsync(h_sc, sc, sizeof(SchurScal), cudaMemcpyDeviceToHost, st));
-      GSLS_CUDA(cudaStreamSynchronize(st));
-      if (prof) {
-        // per CG iteration: count = iterations of this call
-        float ms = 0.f;
-        GSLS_CUDA(cudaEventElapsedTime(&ms, pe0, pe1));
-        prof_add("schur", h_sc->itr, ms);
-        prof_add("schur_calls", 1, ms);
-        cudaEventDestroy(pe0);
-        cudaEventDestroy(pe1);
-      }
-      if (h_sc->done == 4) {
-        set_error("NS: grid barrier of the Schur-complement CG timed out");
-        return GSLS_ERR_CUDA;
-      }
-    }
+  } else {
+    k_schur_init<XT><<<G, kNT, 0, st>>>(nNo, P, Rs, Ps, part, tk, sc, ls->absTol, ls->relTol,
+                                        ls->mItr);
+    GSLS_CHECK_LAUNCH();
   }
   const int batch = 8;
-  for (; use_kernels;) {
+  while (!windowed) {
     GSLS_CUDA(cudaMemcpyAsync(h_sc, sc, sizeof(SchurScal), cudaMemcpyDeviceToHost, st));
     GSLS_CUDA(cudaStreamSynchronize(st));
     if (h_sc->done) break;
@@ -1111,24 +760,21 @@ static int ns_t(gsls_lhs *lhs, gsls_ls *ls, const VT *Val, double *R, const doub
   auto t0 = std::chrono::steady_clock::now();
   // vectors: Rmi Rm GP MU(nB) U(mI) (3-vectors); Rci Rc Rs Ps SP Pb MP(nB) P(mI) (scalars)
   const size_t l3 = ((size_t)nNo * 3 + 63) & ~(size_t)63, l1 = ((size_t)nNo + 63) & ~(size_t)63;
-  const size_t nvec3 = 5 + (size_t)nB + mI, nvec1 = 6 + (size_t)nB + mI;
+  const size_t nvec3 = 3 + (size_t)nB + mI, nvec1 = 5 + (size_t)nB + mI;
   GSLS_TRY(ws.ns_vec.alloc(sizeof(XT) * (nvec3 * l3 + nvec1 * l1) + 2048 + 2 * sizeof(SchurScal)));
   XT *v3 = ws.ns_vec.as<XT>();
-  XT *Rmi = v3, *Rm = v3 + l3, *GP = v3 + 2 * l3, *GP4 = v3 + 3 * l3;  // GP4: 4 per node
-  XT *MU = v3 + 5 * l3, *U = MU + (size_t)nB * l3;
+  XT *Rmi = v3, *Rm = v3 + l3, *GP = v3 + 2 * l3;
+  XT *MU = v3 + 3 * l3, *U = MU + (size_t)nB * l3;
   XT *v1 = v3 + nvec3 * l3;
   XT *Rci = v1, *Rc = v1 + l1, *Rs = v1 + 2 * l1, *Ps = v1 + 3 * l1, *SP = v1 + 4 * l1;
-  XT *Pb = v1 + 5 * l1, *MP = v1 + 6 * l1, *P = MP + (size_t)nB * l1;
+  XT *MP = v1 + 5 * l1, *P = MP + (size_t)nB * l1;
   SchurScal *sc = reinterpret_cast<SchurScal *>(
       (reinterpret_cast<uintptr_t>(v1 + nvec1 * l1) + 127) & ~(uintptr_t)127);
   double *dsc = reinterpret_cast<double *>(sc + 2);  // 96 doubles: norms and dots
-  GridBar *bar = reinterpret_cast<GridBar *>(dsc + 96);
   const size_t m9 = (size_t)nnz * 9, m3 = (size_t)nnz * 3;
   const size_t m1 = ((size_t)nnz + 15) & ~(size_t)15;
-  GSLS_TRY(ws.ns_mat.alloc(sizeof(VT) * (m9 + 4 * m3 + m1 + 8 * (size_t)nnz) + 256));
+  GSLS_TRY(ws.ns_mat.alloc(sizeof(VT) * (m9 + 3 * m3 + m1) + 256));
   VT *mK = ws.ns_mat.as<VT>(), *mG = mK + m9, *mD = mG + m3, *Gt = mD + m3, *mL = Gt + m3;
-  VT *A1 = reinterpret_cast<VT *>((reinterpret_cast<uintptr_t>(mL + m1) + 63) & ~(uintptr_t)63);
-  VT *A2 = A1 + 4 * (size_t)nnz;
   // the GMRES workspace may grow ws.partials: size it for both up front
   const int Gd = num_sms() * 2;
   const int sD = ls->GM.sD > 0 ? ls->GM.sD : 1;
@@ -1142,8 +788,17 @@ static int ns_t(gsls_lhs *lhs, gsls_ls *ls, const VT *Val, double *R, const doub
   k_ns_split<XT><<<G, kNT, 0, st>>>(nNo, R, Rmi, Rci, Rm, Rc, part, tk, dsc);
   GSLS_CHECK_LAUNCH();
   k_depart<VT><<<grid_for(nnz, G * 4), kNT, 0, st>>>(nnz, Val, lhs->d_tpos.as<int>(), mK, mG, mD, mL,
-                                                      Gt, A1, A2);
+                                                      Gt);
   GSLS_CHECK_LAUNCH();
+  // one launch per Schur CG, unless a block's windows do not fit in shared
+  // memory or coupled faces add a global dot between the two Schur products
+  // (GSLS_SCHUR=kernels: never)
+  static const bool kernels = [] {
+    const char *e = getenv("GSLS_SCHUR");
+    return e && strcmp(e, "kernels") == 0;
+  }();
+  bool windowed = false;
+  if (!kernels && !ws.cpl_on) GSLS_TRY(wschur_pack<VT>(lhs, mG, Gt, mL, &windowed));
   double n2[2];
   GSLS_CUDA(cudaMemcpyAsync(n2, dsc, sizeof(n2), cudaMemcpyDeviceToHost, st));
   GSLS_CUDA(cudaStreamSynchronize(st));
@@ -1176,8 +831,7 @@ static int ns_t(gsls_lhs *lhs, gsls_ls *ls, const VT *Val, double *R, const doub
     part = ws.partials.as<double>();
     k_ns_vs<VT, XT><<<G, kNT, 0, st>>>(nNo, rp, cp, mD, Ui, Rc, Pi, nullptr);
     GSLS_CHECK_LAUNCH();
-    GSLS_TRY((schur_cg<VT, XT>(lhs, &ls->CG, mG, Gt, mL, A1, A2, Pi, Rs, Ps, Pb, SP, GP, GP4, sc,
-                               &h_sc, bar)));
+    GSLS_TRY((schur_cg<VT, XT>(lhs, &ls->CG, mG, Gt, mL, Pi, Rs, Ps, SP, GP, sc, &h_sc, windowed)));
     k_ns_sv<VT, XT><<<G, kNT, 0, st>>>(nNo, rp, cp, mG, Pi, MUiB, Rm, MUiBB, nullptr);
     GSLS_CHECK_LAUNCH();
     GSLS_TRY((gmres_ns<3, VT, XT>(lhs, &ls->GM, mK, MUiBB, Ui)));

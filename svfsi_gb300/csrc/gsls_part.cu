@@ -39,9 +39,10 @@ static bool for_blocks(int nblk, long long work, size_t n, const F &f) {
 }
 
 struct PartHost {
-  int nblk = 0, L = 1, winMax = 0, nslMax = 0, stMax = 0;
+  int nblk = 0, L = 1, winMax = 0, nslMax = 0, stMax = 0, grpMax = 0;
+  long long steps8 = 0;
   bool ok = false;
-  std::vector<int> wbase, sbase, slen, hoff, halo, slotRow, src;
+  std::vector<int> wbase, sst, soff, sbase, slen, hoff, halo, slotRow, src;
   std::vector<unsigned short> lcol;
 };
 
@@ -182,6 +183,22 @@ static void part_host(int nNo, const std::vector<int> &rp, const std::vector<int
     if (steps > (1LL << 31) / 32 - 1) return;
   }
   wbase[wst.size()] = (int)steps;
+  // slices in steps of their own, from multiples of 8
+  H.sst.assign(nS, 0);
+  H.soff.assign((size_t)nS + 1, 0);
+  long long steps8 = 0;
+  std::vector<int> wgr((size_t)nblk * W, 0);
+  for (int b = 0; b < nblk; b++)
+    for (int s = sbase[b]; s < sbase[b + 1]; s++) {
+      const int g = (slen[s] + 7) / 8;
+      H.soff[s] = (int)steps8;
+      steps8 += 8 * g;
+      wgr[(size_t)b * W + (s - sbase[b]) % W] += g;
+      if (steps8 > (1LL << 31) / 32 - 1 || steps8 - H.soff[sbase[b]] > kGrpOff) return;
+    }
+  H.soff[nS] = (int)steps8;
+  H.steps8 = steps8;
+  for (int g : wgr) H.grpMax = std::max(H.grpMax, g);
   // pass 2: halo of each block, sources and window columns of its steps
   std::vector<std::vector<int>> hl(nblk);
   std::vector<int> &src = H.src;
@@ -210,6 +227,7 @@ static void part_host(int nNo, const std::vector<int> &rp, const std::vector<int
     for (int s = sbase[b]; s < sbase[b + 1]; s++) {
       const int w = (s - sbase[b]) % W, st0 = at[w];
       at[w] += slen[s];
+      H.sst[s] = st0;
       for (int g = 0; g < RW; g++) {
         const int i = slotRow[(size_t)s * RW + g];
         const unsigned short me = (unsigned short)((s - sbase[b]) * RW + g);
@@ -263,7 +281,7 @@ static int part_build(gsls_lhs *lhs, RowPart &p) {
   p.ok = H.ok;
   if (H.ok) {
     std::vector<unsigned char> img;
-    img.reserve(sizeof(int) * (H.wbase.size() + H.sbase.size() + H.slen.size() + H.hoff.size() +
+    img.reserve(sizeof(int) * (H.wbase.size() + 2 * H.soff.size() + H.sbase.size() + H.slen.size() + H.hoff.size() +
                                H.halo.size() + H.slotRow.size() + H.src.size()) +
                 2 * H.lcol.size() + 256);
     p.off[0] = append(img, H.wbase);
@@ -274,6 +292,8 @@ static int part_build(gsls_lhs *lhs, RowPart &p) {
     p.off[5] = append(img, H.slotRow);
     p.off[6] = append(img, H.src);
     p.off[7] = append(img, H.lcol);
+    p.off[8] = append(img, H.sst);
+    p.off[9] = append(img, H.soff);
     GSLS_TRY(p.buf.alloc(img.size() + 16));
     GSLS_CUDA(cudaMemcpyAsync(p.buf.p, img.data(), img.size(), cudaMemcpyHostToDevice,
                               lhs->stream));
@@ -282,6 +302,9 @@ static int part_build(gsls_lhs *lhs, RowPart &p) {
     p.winMax = H.winMax;
     p.nslMax = H.nslMax;
     p.stMax = H.stMax;
+    p.grpMax = H.grpMax;
+    p.nS = (int)H.slen.size();
+    p.steps8 = H.steps8;
     p.slots = (long long)H.slotRow.size();
     p.steps = (long long)H.wbase.back();
   }
@@ -312,12 +335,17 @@ PartArgs part_args(const RowPart &p) {
   a.halo = ints(4);
   a.slotRow = ints(5);
   a.src = ints(6);
+  a.sst = ints(8);
+  a.soff = ints(9);
   a.lcol = reinterpret_cast<const unsigned short *>(d + p.off[7]);
   a.nblk = p.nblk;
   a.L = p.L;
   a.winMax = p.winMax;
   a.nslMax = p.nslMax;
   a.stMax = p.stMax;
+  a.grpMax = p.grpMax;
+  a.nS = p.nS;
+  a.nsteps8 = p.steps8;
   a.nslots = p.slots;
   a.nsteps = p.steps;
   return a;

@@ -28,6 +28,8 @@ constexpr int kPartMaxBlocks = 256;
 
 struct PartArgs {
   const int *wbase;   // first step of each (block, warp), nblk * kPartWarps + 1
+  const int *sst;     // first step of each slice
+  const int *soff;    // the same with every slice starting at a multiple of 8
   const int *sbase;   // first slice of each block, nblk + 1
   const int *slen;    // steps of each slice (>= 1)
   const int *hoff;    // halo offsets, nblk + 1
@@ -36,8 +38,9 @@ struct PartArgs {
   const int *src;     // CSR block of each (step, lane) or -1
   const unsigned short *lcol;  // window index of each (step, lane)
   int nblk, L;
-  int winMax, nslMax, stMax;  // largest window, slices and steps of a warp
-  long long nslots, nsteps;
+  int winMax, nslMax, stMax;  // largest window, slices of a block, steps of a warp
+  int nS, grpMax;             // all slices; groups of 8 steps of a warp
+  long long nslots, nsteps, nsteps8;  // slots; steps, and those of soff
 };
 
 // Partition of the lhs over at most num_sms() blocks; built on the host once
@@ -115,6 +118,33 @@ __device__ __forceinline__ void for_nodes(int n, const Ld &load, const Use &use)
     for (int u = 0; u < B; u++)
       if (k0 + u * kPartThreads < n) use(k0 + u * kPartThreads, v[u]);
   }
+}
+
+// Groups of G (at most 8) steps that never hold steps of two slices, as a
+// table of each warp in shared memory: the group's first
+// step (soff) relative to the block's, the steps of it that belong to the
+// slice, and whether it is the slice's first or last.  Written by the warp's lane 0
+// (table of at least nslMax / kPartWarps + 1 + grpMax * 8 / G entries); the
+// number of groups on every lane.
+constexpr int kGrpOff = (1 << 20) - 1, kGrpLast = 1 << 24, kGrpFirst = 1 << 25;
+__device__ __forceinline__ int grp_valid(int e) { return (e >> 20) & 15; }
+__host__ __device__ __forceinline__ int grp_cap(int nslMax, int grpMax, int G) {
+  return nslMax / kPartWarps + 1 + grpMax * (8 / G);
+}
+template <int G>
+static __device__ __noinline__ int part_groups(const int *__restrict__ soff,
+                                               const int *__restrict__ slen, int nsl, int w,
+                                               int *tab) {
+  int n = 0;
+  if ((threadIdx.x & 31) == 0)
+    for (int s = w; s < nsl; s += kPartWarps) {
+      const int len = __ldg(slen + s), at = __ldg(soff + s) - __ldg(soff);
+      for (int t = 0; t < len; t += G)
+        tab[n++] = (at + t) | min(G, len - t) << 20 | (t + G >= len ? kGrpLast : 0) |
+                   (t == 0 ? kGrpFirst : 0);
+    }
+  __syncwarp();
+  return __shfl_sync(0xffffffffu, n, 0);
 }
 
 }  // namespace gsls
