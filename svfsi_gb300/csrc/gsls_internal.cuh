@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -164,6 +165,8 @@ struct Workspace {
   unsigned long long wcg_serial = 0;  // preconditioning whose matrix the stream holds
   const void *wcg_val = nullptr;      // (and the array it was packed from)
   int wcg_key = 0;                    // block size and value type of the stream
+  DevBuf x32;         // FP32 copy of the vector of gsls_spmv_dev
+  std::mutex x32_mu;  // held while the copy and the product that reads it are enqueued
   DevBuf partials;    // double[grid * 64]
   DevBuf ticket;      // unsigned[8]
   DevBuf scal;        // KrylovScalars; then GridRedBuf

@@ -1143,34 +1143,77 @@ int solve_dev(gsls_lhs *lhs, gsls_ls *ls, int dof, double *dRi, void *dVal, int 
 #undef GSLS_SOLVE_CASE
 }
 
+// LN groups of D lanes per row, the most (of 1, 2, 4; 1, 2 for D = 3) that half
+// the resident warps cover in one pass; scalar rows at least 2, whose lanes
+// would otherwise walk 32 rows apart (20^3 cube, 9,261 scalar rows: 13.9 ->
+// 12.8 us a call with 4, most of it launch and synchronisation)
+template <int D, int VD, class VT, class XT>
+static int spmv_ln(gsls_lhs *lhs, const VT *Val, const XT *x, double *y, bool after) {
+  const int nNo = lhs->nNo;
+  const long long half = 32LL * num_sms();
+  int LN = D == 3 ? 2 : 4;
+  while (LN > (D == 1 ? 2 : 1) && (long long)nNo * LN * D > half * 32) LN /= 2;
+  const long long rows = LN == 4 ? 32 / D / 4 : LN == 2 ? 32 / D / 2 : 32 / D;
+  const long long warps = ((long long)nNo + rows - 1) / rows;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = after ? 1 : 0;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)std::min<long long>((warps + 7) / 8, 8LL * num_sms()));
+  cfg.blockDim = dim3(256);
+  cfg.stream = lhs->stream;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  const int *rp = lhs->d_rowPtr.as<int>(), *cp = lhs->d_colPtr.as<int>();
+  if constexpr (D != 3)
+    if (LN == 4)
+      GSLS_CUDA(cudaLaunchKernelEx(&cfg, k_spmv_ln<D, 4, VD, VT, XT, double>, nNo, rp, cp, Val, x, y));
+  if (LN == 2)
+    GSLS_CUDA(cudaLaunchKernelEx(&cfg, k_spmv_ln<D, 2, VD, VT, XT, double>, nNo, rp, cp, Val, x, y));
+  if constexpr (D != 1)
+    if (LN == 1)
+      GSLS_CUDA(cudaLaunchKernelEx(&cfg, k_spmv_ln<D, 1, VD, VT, XT, double>, nNo, rp, cp, Val, x, y));
+  GSLS_CHECK_LAUNCH();
+  return GSLS_OK;
+}
+
+template <int D>
+static int spmv_t(gsls_lhs *lhs, const void *dVal, bool mixed, const double *x, double *y) {
+  if (!mixed) return spmv_ln<D, D>(lhs, (const double *)dVal, x, y, false);
+  // FP32 values: x is rounded to FP32 once in front of the product where the
+  // rounding in the gathers would take longer than a launch (an FP64 -> FP32
+  // conversion per matrix value, ~0.55 T/s: 2.5 us at 2^21 / 1.5 values; the
+  // 3x3 beam of 47 M values 119 -> 68 us, of which 32 us are its bytes at the
+  // HBM copy rate)
+  if ((long long)lhs->nnz * D * D < (2 << 20))
+    return spmv_ln<D, D>(lhs, (const float *)dVal, x, y, false);
+  constexpr int VD = VStride<D, float>::v;
+  std::lock_guard<std::mutex> lk(lhs->ws.x32_mu);
+  GSLS_TRY(lhs->ws.x32.alloc(sizeof(float) * (size_t)lhs->nNo * VD));
+  float *xf = lhs->ws.x32.as<float>();
+  k_x32<D, VD><<<blocks_for(lhs->nNo, num_sms() * 8), 256, 0, lhs->stream>>>(lhs->nNo, x, xf);
+  GSLS_CHECK_LAUNCH();
+  return spmv_ln<D, VD>(lhs, (const float *)dVal, (const float *)xf, y, true);
+}
+
 int spmv_launch(gsls_lhs *lhs, int dof, const void *dVal, int val_prec, const void *dx, void *dy,
                 int xprec) {
   (void)xprec;
-  cudaStream_t st = lhs->stream;
-  const int G = lhs->grid;
   const bool mixed = (val_prec == GSLS_PREC_MIXED);
-#define GSLS_SPMV_CASE(DV)                                                                    \
-  case DV:                                                                                    \
-    if (mixed)                                                                                \
-      k_spmv<DV, float, double, double><<<G, kThreads, 0, st>>>(                              \
-          lhs->nNo, lhs->d_rowPtr.as<int>(), lhs->d_colPtr.as<int>(), (const float *)dVal,     \
-          (const double *)dx, (double *)dy);                                                  \
-    else                                                                                      \
-      k_spmv<DV, double, double, double><<<G, kThreads, 0, st>>>(                             \
-          lhs->nNo, lhs->d_rowPtr.as<int>(), lhs->d_colPtr.as<int>(), (const double *)dVal,    \
-          (const double *)dx, (double *)dy);                                                  \
-    break;
+  const double *x = (const double *)dx;
+  double *y = (double *)dy;
   switch (dof) {
-    GSLS_SPMV_CASE(1)
-    GSLS_SPMV_CASE(2)
-    GSLS_SPMV_CASE(3)
-    GSLS_SPMV_CASE(4)
+    case 1:
+      return spmv_t<1>(lhs, dVal, mixed, x, y);
+    case 2:
+      return spmv_t<2>(lhs, dVal, mixed, x, y);
+    case 3:
+      return spmv_t<3>(lhs, dVal, mixed, x, y);
+    case 4:
+      return spmv_t<4>(lhs, dVal, mixed, x, y);
     default:
       return GSLS_ERR_UNSUPPORTED;
   }
-#undef GSLS_SPMV_CASE
-  GSLS_CHECK_LAUNCH();
-  return GSLS_OK;
 }
 
 }  // namespace gsls

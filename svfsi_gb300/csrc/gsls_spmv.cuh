@@ -88,11 +88,13 @@ struct GatherDir {
   }
 };
 
-// y_r of block row i for lane component r
-template <int D, class VT, class AT, class G>
+// y_r of block row i for lane component r (LN > 1: of its blocks part, part +
+// LN, ...)
+template <int D, class VT, class AT, int LN = 1, class G>
 __device__ __forceinline__ AT spmv_row_comp(int i, int r, const int *__restrict__ rowPtr,
                                             const int *__restrict__ colPtr,
-                                            const VT *__restrict__ Val, const G &g) {
+                                            const VT *__restrict__ Val, const G &g,
+                                            int part = 0) {
   constexpr int DD = D * D;
   const int rs = __ldg(rowPtr + i), re = __ldg(rowPtr + i + 1);
   const VT *__restrict__ v = Val + (size_t)rs * DD + r * D;
@@ -100,15 +102,15 @@ __device__ __forceinline__ AT spmv_row_comp(int i, int r, const int *__restrict_
   // U blocks per step: column loads, value loads and gathers of all U
   // blocks are issued before the first FMA
   constexpr int U = 4;
-  for (int j = rs; j < re; j += U) {
+  for (int j = rs + part; j < re; j += U * LN) {
     int cc[U];
 #pragma unroll
-    for (int u = 0; u < U; u++) cc[u] = (j + u < re) ? __ldg(colPtr + j + u) : -1;
+    for (int u = 0; u < U; u++) cc[u] = (j + u * LN < re) ? __ldg(colPtr + j + u * LN) : -1;
     AT a[U][D], xg[U][D];
 #pragma unroll
     for (int u = 0; u < U; u++) {
       if (cc[u] >= 0) {
-        load_row_seg<D, VT, AT>(v + (size_t)(j + u - rs) * DD, a[u]);
+        load_row_seg<D, VT, AT>(v + (size_t)(j + u * LN - rs) * DD, a[u]);
         g.get(cc[u], xg[u]);
       } else {
 #pragma unroll
@@ -145,6 +147,44 @@ __global__ void __launch_bounds__(256) k_spmv(int nNo, const int *__restrict__ r
     if (grp < RPW && i < nNo)
       y[(size_t)i * D + r] = YT(spmv_row_comp<D, VT, AT>(i, r, rowPtr, colPtr, Val, g));
   }
+}
+
+// y = K x with LN groups of D lanes per block row (blocks strided by LN, four
+// of each group's loads in flight); the groups' sums are added by shuffles.
+// A small system has too few rows to fill the SMs with a group each, and a
+// row is then a chain of ~4 rounds of dependent loads instead of one or two.
+template <int D, int LN, int VD, class VT, class XT, class YT>
+__global__ void __launch_bounds__(256) k_spmv_ln(int nNo, const int *__restrict__ rowPtr,
+                                                 const int *__restrict__ colPtr,
+                                                 const VT *__restrict__ Val,
+                                                 const XT *__restrict__ x, YT *__restrict__ y) {
+  cudaGridDependencySynchronize();
+  using AT = typename AccOf<VT>::T;
+  constexpr int NG = 32 / D, RPW = NG / LN;
+  const int lane = threadIdx.x & 31, grp = lane / D, r = lane - grp * D;
+  const int slot = grp / LN, part = grp - slot * LN;
+  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int nwarps = (gridDim.x * blockDim.x) >> 5;
+  GatherX<D, XT, AT, VD> g{x};
+  for (int base = warp * RPW; base < nNo; base += nwarps * RPW) {
+    const int i = base + slot;
+    const bool on = slot < RPW && i < nNo;
+    AT s = on ? spmv_row_comp<D, VT, AT, LN>(i, r, rowPtr, colPtr, Val, g, part) : AT(0);
+#pragma unroll
+    for (int o = LN / 2; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o * D);
+    if (on && part == 0) y[(size_t)i * D + r] = YT(s);
+  }
+}
+
+// x in FP32 at node stride VD: the gathers of an FP32 matrix read it ~15 times
+// per entry, and an FP64 -> FP32 conversion runs at the FP64 rate
+template <int D, int VD>
+__global__ void __launch_bounds__(256) k_x32(int nNo, const double *__restrict__ x,
+                                             float *__restrict__ xf) {
+  cudaTriggerProgrammaticLaunchCompletion();
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nNo; i += gridDim.x * blockDim.x)
+#pragma unroll
+    for (int c = 0; c < D; c++) xf[(size_t)i * VD + c] = (float)x[(size_t)i * D + c];
 }
 
 __device__ __forceinline__ float warp_sum_f(float v) {
