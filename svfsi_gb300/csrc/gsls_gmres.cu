@@ -77,8 +77,9 @@ __global__ void k_gm_scale(size_t n, XT *__restrict__ u, const double *normp) {
 }
 
 // SpMV that is skipped once the Arnoldi loop is done; rev: rows walked from
-// the end (zig-zag order across Arnoldi steps, zigzag_on)
-template <int D, class VT, class XT>
+// the end (zig-zag order across Arnoldi steps, zigzag_on).  LN = 2: two groups
+// of D lanes per row, for systems whose rows do not fill the SMs.
+template <int D, int LN, class VT, class XT>
 __global__ void __launch_bounds__(kT) k_gm_spmv(int nNo, const int *__restrict__ rowPtr,
                                                 const int *__restrict__ colPtr,
                                                 const VT *__restrict__ Val,
@@ -86,16 +87,30 @@ __global__ void __launch_bounds__(kT) k_gm_spmv(int nNo, const int *__restrict__
                                                 const GmresCtl *ctl, int rev) {
   if (*(volatile const int *)&ctl->done) return;
   using AT = typename AccOf<VT>::T;
-  constexpr int RPW = 32 / D;
+  constexpr int RPW = 32 / D / LN;
   const int lane = threadIdx.x & 31, grp = lane / D, r = lane - grp * D;
+  const int slot = grp / LN, part = grp - slot * LN;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
   GatherX<D, XT, AT> g{x};
   for (int base = warp * RPW; base < nNo; base += nwarps * RPW) {
-    const int i = rev ? nNo - 1 - (base + grp) : base + grp;
-    if (grp < RPW && i >= 0 && i < nNo)
-      y[(size_t)i * D + r] = XT(spmv_row_comp<D, VT, AT>(i, r, rowPtr, colPtr, Val, g));
+    const int i = rev ? nNo - 1 - (base + slot) : base + slot;
+    const bool on = slot < RPW && i >= 0 && i < nNo;
+    AT s = on ? spmv_row_comp<D, VT, AT, LN>(i, r, rowPtr, colPtr, Val, g, part) : AT(0);
+    if constexpr (LN == 2) s += __shfl_down_sync(0xffffffffu, s, D);
+    if (on && part == 0) y[(size_t)i * D + r] = XT(s);
   }
+}
+template <int D, class VT, class XT>
+static void gm_spmv(gsls_lhs *lhs, const VT *Val, const XT *x, XT *y, const GmresCtl *ctl,
+                    int rev) {
+  const int nNo = lhs->nNo, G = lhs->grid;
+  const int *rp = lhs->d_rowPtr.as<int>(), *cp = lhs->d_colPtr.as<int>();
+  // two groups per row while they fit on the SMs at once (2048 threads each)
+  if ((long long)nNo * 2 * D <= 2048LL * num_sms())
+    k_gm_spmv<D, 2, VT, XT><<<G, kT, 0, lhs->stream>>>(nNo, rp, cp, Val, x, y, ctl, rev);
+  else
+    k_gm_spmv<D, 1, VT, XT><<<G, kT, 0, lhs->stream>>>(nNo, rp, cp, Val, x, y, ctl, rev);
 }
 
 // 16-byte vectors of the Krylov type: four FP32 or two FP64 values.  Basis
@@ -178,66 +193,114 @@ __global__ void __launch_bounds__(kT) k_gm_multidot(size_t n, const XT *__restri
         if (two) acc_b = fma(basis[ld * (j + 1) + k], v[k], acc_b);
       }
     }
-    const double a = warp_sum(double(acc_a));
-    const double b = warp_sum(double(acc_b));
-    if (lane == 0) {
-      partials[(size_t)j * gridDim.x + blockIdx.x] = a;
-      if (two) partials[(size_t)(j + 1) * gridDim.x + blockIdx.x] = b;
-    }
+    // both sums in five FP64 adds: after the first exchange the lower half of
+    // the warp carries the one, the upper half the other
+    const double lo = double(lane < 16 ? acc_a : acc_b), hi = double(lane < 16 ? acc_b : acc_a);
+    double v2 = lo + __shfl_xor_sync(0xffffffffu, hi, 16);
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) v2 += __shfl_xor_sync(0xffffffffu, v2, o);
+    if (lane == 0) partials[(size_t)j * gridDim.x + blockIdx.x] = v2;
+    if (lane == 16 && two) partials[(size_t)(j + 1) * gridDim.x + blockIdx.x] = v2;
   }
 }
 
-// Column sums of the multi-dot partials: one block per j (deterministic).
-__global__ void k_gm_colsum(int grid, const double *partials, double *h, const GmresCtl *ctl) {
-  if (*(volatile const int *)&ctl->done) return;
+// Norm + Givens rotation for column i (1-based) by one warp.  pyth: hcol[i]
+// holds v.v and the norm is the Pythagorean sqrt|v.v - sum h_j^2|; else
+// hcol[i] already holds |v - sum h_j u_j|^2.  hraw[0..i] receives the
+// unrotated column for the Gram-Schmidt update.
+// The rotations of a column are the recurrence v_j = -s v_{j-1} + c h_j, with
+// the rotated entry h'_{j-1} = c v_{j-1} + s h_j: 32 of them at a time as a
+// scan of affine maps (an FP64 FMA takes ~150 cycles, and one thread that
+// walks the column through memory took 12.5 us at 25 columns, this 4 us).
+struct GivensArgs {
+  int sD;
+  double *H, *hcol, *hraw, *c, *s, *err;
+  GmresCtl *ctl;
+};
+static __device__ void gm_givens(const GivensArgs &G, bool pyth) {
+  const int lane = threadIdx.x & 31;
+  const int i = G.ctl->i;
+  double *h = G.H + (size_t)(i - 1) * (G.sD + 1);
+  double sq = 0.0;
+  double v = __ldcg(G.hcol);  // v_0
+  for (int j0 = 0; j0 < i; j0 += 32) {
+    // element j = j0 + lane of the column; its rotation (with j + 1) uses c[j], s[j]
+    const int j = j0 + lane;
+    const double hj = j < i ? __ldcg(G.hcol + j) : 0.0;
+    if (j < i) {
+      G.hraw[j] = hj;
+      sq = fma(hj, hj, sq);
+    }
+    const bool rot = j < i - 1;
+    const double c = rot ? G.c[j] : 1.0, s = rot ? G.s[j] : 0.0;
+    const double hn = rot ? __ldcg(G.hcol + j + 1) : 0.0;
+    // v_{j+1} = A v_j + B, scanned
+    double A = rot ? -s : 1.0, B = rot ? c * hn : 0.0;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const double Ap = __shfl_up_sync(0xffffffffu, A, o), Bp = __shfl_up_sync(0xffffffffu, B, o);
+      if (lane >= o) {
+        B = fma(A, Bp, B);
+        A = A * Ap;
+      }
+    }
+    const double vn = fma(A, v, B);  // v_{j+1}
+    double vj = __shfl_up_sync(0xffffffffu, vn, 1);
+    if (lane == 0) vj = v;
+    if (rot) h[j] = fma(c, vj, s * hn);
+    v = __shfl_sync(0xffffffffu, vn, 31);
+  }
+  // v is the rotated h_{i-1}; the new subdiagonal entry
+  double hi = __ldcg(G.hcol + i);
+  if (pyth) hi -= warp_sum(sq);
+  if (lane == 0) {
+    hi = sqrt(fabs(hi));
+    G.hraw[i] = hi;
+    const double x = v * v + hi * hi, r = rsqrt(x);
+    const double tmp = x * r, ci = v * r, si = hi * r;
+    G.c[i - 1] = ci;
+    G.s[i - 1] = si;
+    h[i - 1] = tmp;
+    h[i] = 0.0;
+    const double e0 = G.err[i - 1], e1 = -si * e0;
+    G.err[i] = e1;
+    G.err[i - 1] = ci * e0;
+    GmresCtl *ctl = G.ctl;
+    ctl->last_i = i;
+    if (!isfinite(e1) || !isfinite(hi) || hi == 0.0) {
+      // breakdown: h(i+1,i) = 0 or non-finite
+      ctl->nan = (!isfinite(e1) || !isfinite(hi)) ? 1 : 0;
+      ctl->conv = ctl->nan ? 0 : 1;
+      ctl->done = 1;
+    } else if (fabs(e1) < ctl->eps) {
+      ctl->conv = 1;
+      ctl->done = 1;
+    }
+    ctl->i = i + 1;
+    if (i >= G.sD) ctl->done = 1;
+  }
+}
+
+// Column sums of the multi-dot partials: one block per j (deterministic);
+// rotate: the last block to finish rotates the column.
+__global__ void __launch_bounds__(kT) k_gm_colsum(int grid, const double *partials, GivensArgs G,
+                                                  unsigned *ticket, int rotate) {
+  if (*(volatile const int *)&G.ctl->done) return;
   __shared__ double sh[32];
+  __shared__ int last;
   const int j = blockIdx.x;
   double s = 0.0;
   for (int b = threadIdx.x; b < grid; b += blockDim.x) s += partials[(size_t)j * grid + b];
   s = block_sum(s, sh);
-  if (threadIdx.x == 0) h[j] = s;
-}
-
-// Norm + Givens rotation for column i (1-based), one thread.  pyth: hcol[i]
-// holds v.v and the norm is the Pythagorean sqrt|v.v - sum h_j^2|; else
-// hcol[i] already holds |v - sum h_j u_j|^2.  hraw[0..i] receives the
-// unrotated column for the Gram-Schmidt update.
-__global__ void k_gm_givens(int sD, double *H, const double *hcol, double *hraw, double *c,
-                            double *s, double *err, GmresCtl *ctl, int pyth) {
-  if (ctl->done) return;
-  const int i = ctl->i;
-  double *h = H + (size_t)(i - 1) * (sD + 1);
-  for (int j = 0; j <= i; j++) h[j] = hcol[j];
-  for (int j = 0; j < i; j++) {
-    hraw[j] = h[j];
-    if (pyth) h[i] = h[i] - h[j] * h[j];
+  if (threadIdx.x == 0) {
+    __stcg(G.hcol + j, s);
+    if (rotate) last = atomic_add_acq_rel(ticket, 1u) == gridDim.x - 1;
   }
-  h[i] = sqrt(fabs(h[i]));
-  hraw[i] = h[i];
-  for (int j = 1; j <= i - 1; j++) {
-    const double tmp = c[j - 1] * h[j - 1] + s[j - 1] * h[j];
-    h[j] = -s[j - 1] * h[j - 1] + c[j - 1] * h[j];
-    h[j - 1] = tmp;
-  }
-  const double tmp = sqrt(h[i - 1] * h[i - 1] + h[i] * h[i]);
-  c[i - 1] = h[i - 1] / tmp;
-  s[i - 1] = h[i] / tmp;
-  h[i - 1] = tmp;
-  h[i] = 0.0;
-  err[i] = -s[i - 1] * err[i - 1];
-  err[i - 1] = c[i - 1] * err[i - 1];
-  ctl->last_i = i;
-  if (!isfinite(err[i]) || !isfinite(hraw[i]) || hraw[i] == 0.0) {
-    // breakdown: h(i+1,i) = 0 or non-finite
-    ctl->nan = (!isfinite(err[i]) || !isfinite(hraw[i])) ? 1 : 0;
-    ctl->conv = ctl->nan ? 0 : 1;
-    ctl->done = 1;
-  } else if (fabs(err[i]) < ctl->eps) {
-    ctl->conv = 1;
-    ctl->done = 1;
-  }
-  ctl->i = i + 1;
-  if (i >= sD) ctl->done = 1;
+  if (!rotate) return;
+  __syncthreads();
+  if (!last) return;
+  if (threadIdx.x == 0) *ticket = 0u;
+  if (threadIdx.x < 32) gm_givens(G, true);
 }
 
 // u_{i+1} = (u_{i+1} - sum_j hraw_j u_j) / hraw_i, one 16-byte group per
@@ -261,7 +324,7 @@ __global__ void __launch_bounds__(kT) k_gm_orth(size_t n, XT *__restrict__ basis
   const size_t nt = (size_t)gridDim.x * blockDim.x;
   for (size_t q = t0; q < nq; q += nt) {
     VT4 acc = reinterpret_cast<const VT4 *>(v)[q];
-#pragma unroll 4
+#pragma unroll 8
     for (int j = 0; j < i; j++) V::axpy(hs[j], reinterpret_cast<const VT4 *>(basis + ld * j)[q], acc);
     V::scale(acc, inv);
     reinterpret_cast<VT4 *>(v)[q] = acc;
@@ -274,15 +337,16 @@ __global__ void __launch_bounds__(kT) k_gm_orth(size_t n, XT *__restrict__ basis
 }
 
 // FP32 basis: u_{i+1} -= sum_{j<i} h_j u_j (h_j from the multi-dot, before
-// the Givens kernel of the step) and |u_{i+1}|^2 -> hcol[i], a deterministic
+// the rotation of the step) and |u_{i+1}|^2 -> hcol[i], a deterministic
 // grid sum; each 16-byte group's squares are summed in FP32 and added in
-// FP64.  k_gm_scale_i then divides by the norm once the Givens kernel has
-// accepted the column.
+// FP64.  The last block rotates the column; k_gm_scale_i then divides by the
+// norm.
 template <class XT>
 __global__ void __launch_bounds__(kT) k_gm_orth_nrm(size_t n, XT *__restrict__ basis, size_t ld,
-                                                    double *__restrict__ hcol, const GmresCtl *ctl,
-                                                    int i, double *partials, unsigned *ticket) {
-  if (*(volatile const int *)&ctl->done) return;
+                                                    GivensArgs G, int i, double *partials,
+                                                    unsigned *ticket) {
+  if (*(volatile const int *)&G.ctl->done) return;
+  const double *hcol = G.hcol;
   using V = Vec16<XT>;
   using VT4 = typename V::T;
   constexpr int L = V::L;
@@ -297,7 +361,7 @@ __global__ void __launch_bounds__(kT) k_gm_orth_nrm(size_t n, XT *__restrict__ b
   double nrm = 0.0;
   for (size_t q = t0; q < nq; q += nt) {
     VT4 acc = reinterpret_cast<const VT4 *>(v)[q];
-#pragma unroll 4
+#pragma unroll 8
     for (int j = 0; j < i; j++) V::axpy(hs[j], reinterpret_cast<const VT4 *>(basis + ld * j)[q], acc);
     reinterpret_cast<VT4 *>(v)[q] = acc;
     nrm += double(V::dot(acc, acc, XT(0)));
@@ -310,10 +374,14 @@ __global__ void __launch_bounds__(kT) k_gm_orth_nrm(size_t n, XT *__restrict__ b
   }
   const double bs = block_sum(nrm, sh);
   double tot;
-  if (grid_reduce_last<1>(&bs, partials, ticket, &tot, sh) && threadIdx.x == 0) hcol[i] = tot;
+  if (grid_reduce_last<1>(&bs, partials, ticket, &tot, sh)) {
+    if (threadIdx.x == 0) __stcg(G.hcol + i, tot);
+    __syncthreads();
+    if (threadIdx.x < 32) gm_givens(G, false);
+  }
 }
 
-// u_{i+1} /= h_{i+1,i} after the Givens kernel of step i (FP32 basis)
+// u_{i+1} /= h_{i+1,i} after the rotation of step i (FP32 basis)
 template <class XT>
 __global__ void k_gm_scale_i(size_t n, XT *__restrict__ basis, size_t ld,
                              const double *__restrict__ hraw, const GmresCtl *ctl, int i) {
@@ -325,15 +393,25 @@ __global__ void k_gm_scale_i(size_t n, XT *__restrict__ basis, size_t ld,
     v[k] = v[k] * inv;
 }
 
-// Back substitution y = H(1:i,1:i)^-1 err(1:i), one thread.
-__global__ void k_gm_backsub(int sD, const double *H, const double *err, double *y,
-                             const GmresCtl *ctl) {
+// Back substitution y = H(1:i,1:i)^-1 err(1:i), one block: the reciprocals of
+// the diagonal at once, then column by column (one thread that walked H
+// through memory, with a division per row, took 144 us at i = 47)
+__global__ void __launch_bounds__(kT) k_gm_backsub(int sD, const double *H, const double *err,
+                                                   double *y, const GmresCtl *ctl) {
+  __shared__ double sy[512], sr[512];
   int i = ctl->last_i;
   if (i > sD) i = sD;
-  for (int j = 0; j < i; j++) y[j] = err[j];
-  for (int j = i; j >= 1; j--) {
-    for (int k = j + 1; k <= i; k++) y[j - 1] -= H[(size_t)(k - 1) * (sD + 1) + (j - 1)] * y[k - 1];
-    y[j - 1] /= H[(size_t)(j - 1) * (sD + 1) + (j - 1)];
+  for (int j = threadIdx.x; j < i; j += blockDim.x) {
+    sy[j] = err[j];
+    sr[j] = 1.0 / H[(size_t)j * (sD + 1) + j];
+  }
+  __syncthreads();
+  for (int k = i - 1; k >= 0; k--) {
+    const double yk = sy[k] * sr[k];
+    for (int j = threadIdx.x; j < k; j += blockDim.x)
+      sy[j] = fma(-H[(size_t)k * (sD + 1) + j], yk, sy[j]);
+    if (threadIdx.x == 0) y[k] = yk;
+    __syncthreads();
   }
 }
 
@@ -429,6 +507,7 @@ static int gmres_loop(gsls_lhs *lhs, gsls_sub_ls *ls, const VT *Val, const XT *R
   XT *basis = ws.basis.as<XT>();
   double *part = ws.partials.as<double>();
   unsigned *tk = ws.ticket.as<unsigned>();
+  const GivensArgs giv{sD, H, hcol, hraw, cc, ss, err, ctl};
   *early = false;
   GSLS_CUDA(cudaMemsetAsync(X, 0, sizeof(XT) * nv, st));
   GmresCtl hc;
@@ -440,8 +519,7 @@ static int gmres_loop(gsls_lhs *lhs, gsls_sub_ls *ls, const VT *Val, const XT *R
     hc.i = 1;
     GSLS_CUDA(cudaMemcpyAsync(ctl, &hc, sizeof(hc), cudaMemcpyHostToDevice, st));
     if (l > 1) {
-      k_gm_spmv<D, VT, XT><<<G, kT, 0, st>>>(nNo, lhs->d_rowPtr.as<int>(),
-                                             lhs->d_colPtr.as<int>(), Val, X, u1, ctl, 0);
+      gm_spmv<D, VT, XT>(lhs, Val, X, u1, ctl, 0);
       GSLS_CHECK_LAUNCH();
       launch_addbcmul<XT>(lhs, 0, D, X, u1, &ctl->done);
     }
@@ -486,9 +564,7 @@ static int gmres_loop(gsls_lhs *lhs, gsls_sub_ls *ls, const VT *Val, const XT *R
         const int i = i_next;
         XT *ui = basis + ld * (i - 1), *ui1 = basis + ld * i;
         if (prof) cudaEventRecord(prof_event(0), st);
-        k_gm_spmv<D, VT, XT><<<G, kT, 0, st>>>(nNo, lhs->d_rowPtr.as<int>(),
-                                               lhs->d_colPtr.as<int>(), Val, ui, ui1, ctl,
-                                               zigzag_on() & i);
+        gm_spmv<D, VT, XT>(lhs, Val, ui, ui1, ctl, zigzag_on() & i);
         GSLS_CHECK_LAUNCH();
         if (prof) cudaEventRecord(prof_event(1), st);
         if (ws.cpl_on) {
@@ -499,20 +575,16 @@ static int gmres_loop(gsls_lhs *lhs, gsls_sub_ls *ls, const VT *Val, const XT *R
           // h_j for j < i, then the orthogonalised vector and its norm
           k_gm_multidot<XT><<<Gd, kT, 0, st>>>(nv, basis, ld, i, ui1, part, ctl);
           GSLS_CHECK_LAUNCH();
-          k_gm_colsum<<<i, kT, 0, st>>>(Gd, part, hcol, ctl);
+          k_gm_colsum<<<i, kT, 0, st>>>(Gd, part, giv, tk, 0);
           GSLS_CHECK_LAUNCH();
-          k_gm_orth_nrm<XT><<<G, kT, 0, st>>>(nv, basis, ld, hcol, ctl, i, part, tk);
-          GSLS_CHECK_LAUNCH();
-          k_gm_givens<<<1, 1, 0, st>>>(sD, H, hcol, hraw, cc, ss, err, ctl, 0);
+          k_gm_orth_nrm<XT><<<G, kT, 0, st>>>(nv, basis, ld, giv, i, part, tk);
           GSLS_CHECK_LAUNCH();
           k_gm_scale_i<XT><<<G, kT, 0, st>>>(nv, basis, ld, hraw, ctl, i);
           GSLS_CHECK_LAUNCH();
         } else {
           k_gm_multidot<XT><<<Gd, kT, 0, st>>>(nv, basis, ld, i + 1, ui1, part, ctl);
           GSLS_CHECK_LAUNCH();
-          k_gm_colsum<<<i + 1, kT, 0, st>>>(Gd, part, hcol, ctl);
-          GSLS_CHECK_LAUNCH();
-          k_gm_givens<<<1, 1, 0, st>>>(sD, H, hcol, hraw, cc, ss, err, ctl, 1);
+          k_gm_colsum<<<i + 1, kT, 0, st>>>(Gd, part, giv, tk, 1);
           GSLS_CHECK_LAUNCH();
           k_gm_orth<XT><<<G, kT, 0, st>>>(nv, basis, ld, hraw, ctl, i);
           GSLS_CHECK_LAUNCH();
@@ -537,7 +609,7 @@ static int gmres_loop(gsls_lhs *lhs, gsls_sub_ls *ls, const VT *Val, const XT *R
       return GSLS_ERR_NAN;
     }
     ls->itr += hc.last_i;
-    k_gm_backsub<<<1, 1, 0, st>>>(sD, H, err, y, ctl);
+    k_gm_backsub<<<1, kT, 0, st>>>(sD, H, err, y, ctl);
     GSLS_CHECK_LAUNCH();
     k_gm_update_x<XT><<<G, kT, 0, st>>>(nv, X, basis, ld, y, ctl);
     GSLS_CHECK_LAUNCH();
