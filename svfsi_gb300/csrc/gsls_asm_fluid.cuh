@@ -12,9 +12,9 @@
 //    uxx, d2u2, es_x, mu_x and rS are zero; the shear rate, mu and mu_g are
 //    element constants, and the viscosity model adds
 //    4 wl mu_g esNx_i(a) esNx_j(b) to Kuu (zero for constant viscosity);
-//  * the residual (u, ud, p, tauM, tauC, tauB, up, rM, lR) is FP64 at every
-//    Gauss point; the tangent runs in TT and is rebuilt per block (a,b) from
-//    eleven per-point factors (tauM, tauC, tauB, u.Nx_a, up.Nx_a):
+//  * the residual (u, ud, p, tauM, tauC, tauB, up, lR) is FP64 at every Gauss
+//    point; the tangent runs in TT and is rebuilt per block (a,b) from factors
+//    accumulated over the points:
 //      Kuu(i,j) = wl [4 mu Nx_i(b)Nx_j(a) + (sum tauC) Nx_i(a)Nx_j(b) + d_ij S_ab]
 //      S_ab     = 4 mu Nx_a.Nx_b + rho amd M_ab
 //                 + sum_g [rho^2 tauM uaNx_a (uNx_b + amd N_b)
@@ -23,6 +23,19 @@
 //      Kpu(j)   =  wl [Ns_a Nx_j(b) + rho Nx_j(a) sum_g tauM (uNx_b + amd N_b)]
 //      Kpp      =  wl (sum tauM) Nx_a.Nx_b
 //    which is the reference's per-point sum with updu = -rho uNx d_ij.
+//
+// The element is bound by the FP64 pipe (0.51 T FMA/s), so its FP64 work is
+// cut by identities of the tet4 rule, which change only the rounding:
+//  * N_a(g) = t + (s - t) d_ag: point values are t sum_a y_a + (s - t) y_g, and
+//    sums over the points of N_a(g) f_g are t sum_g f_g + (s - t) f_a;
+//  * sum_a Nx_a = 0: every quantity f.Nx_a, and every sum of them, is formed
+//    for three nodes and is minus their sum at the fourth;
+//  * x.K.x = sum_{a<3} (x.Nx_a)^2 for the metric tensor K = sum_{a<3} Nx_a Nx_a^T;
+//  * div-free scalars: 1/rho, amd, 4 (ctM/dt)^2 come from the host, tauM,
+//    tauC and tauB from one rsqrt each instead of roots and divisions.
+// FP64 assembly of the h = 0.04 cylinder (371,520 tets): 2.87 ms before, 1.38
+// ms with these and the element buffer (3.3 ms with these and the colour
+// scatter).
 #pragma once
 
 namespace gsls {
@@ -58,22 +71,17 @@ __device__ __forceinline__ void visc_model(const AsmArgs &A, double &gam, double
 // constant-viscosity kernel carries none of its terms
 template <class TT, bool NN>
 __global__ void __launch_bounds__(kAsmThreads) k_asm_fluid(AsmArgs A) {
-  asm_colour_start();
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= A.nColorEl) return;
-  const int e = A.el0 + t;
+  extern __shared__ __align__(16) unsigned char asm_smem[];
+  const EmitAt E = emit_at(A, asm_smem, emit_bytes<TT, 4>(), sizeof(TT) * 256, 4);
+  const int e = A.el0 + min((int)(blockIdx.x * blockDim.x + threadIdx.x), A.nColorEl - 1);
   const int4 nd = A.ien[e];
   const int n4[4] = {nd.x, nd.y, nd.z, nd.w};
   const int tD = A.tDof, s0 = A.s;
 
   // ---- geometry (GNN with ks, FP64, precomputed per mesh): xiX(a,i) = Nx(i,a)
-  double Nx[3][4], K[3][3];
+  double Nx[3][4], kk, trk;
   const double w = c_rule.w * load_geo(A, e, Nx);
-#pragma unroll
-  for (int i = 0; i < 3; i++)
-#pragma unroll
-    for (int j = 0; j < 3; j++)
-      K[i][j] = Nx[i][0] * Nx[j][0] + Nx[i][1] * Nx[j][1] + Nx[i][2] * Nx[j][2];
+  load_metric(A, e, kk, trk);
 
   // ---- nodal values and element-constant gradients (FP64)
   double yl[4][4], al[4][3];
@@ -114,157 +122,216 @@ __global__ void __launch_bounds__(kAsmThreads) k_asm_fluid(AsmArgs A) {
     // ISZERO (MATFUN.f:763-780): |x| < eps^2
     mu_g = (fabs(gam) < 4.930380657631324e-32) ? 0.0 : mu_x / gam;
   }
-  const double rho = A.rho;
-  const double T1c = A.af * A.gam * A.dt;
-  const double amd = A.am / T1c;
-  const double wl = w * T1c, wr = w * rho;
-  const double kT = 4.0 * (A.ctM / A.dt) * (A.ctM / A.dt);
-  double kS = 0.0;
-#pragma unroll
-  for (int i = 0; i < 3; i++)
-#pragma unroll
-    for (int j = 0; j < 3; j++) kS += K[i][j] * K[i][j];
-  kS = A.ctC * kS * (mu / rho) * (mu / rho);
-  const double trK = K[0][0] + K[1][1] + K[2][2];
+  const double rho = A.rho, irho = A.fl_irho;
+  const double wl = w * A.fl_T1, wr = w * rho;
+  const double nu = mu * irho;
+  const double kTS = A.fl_kT + A.ctC * kk * (nu * nu);
+  const double rtrK = rho / trk;
 
-  double lR[4][4];
+  // point values: rt sum_a + rd (value at node g)
+  const double rt = c_rule.N[0][1], rd = c_rule.N[0][0] - c_rule.N[0][1];
+  double uS[3], aS[3];
 #pragma unroll
-  for (int a = 0; a < 4; a++)
-#pragma unroll
-    for (int c = 0; c < 4; c++) lR[a][c] = 0.0;
-  // tangent factors accumulated over the Gauss points
-  const TT rh = TT(rho), md = TT(amd);
-  TT SC = TT(0), ST = TT(0), Q[4], Vc[4], G[4][4];
-#pragma unroll
-  for (int a = 0; a < 4; a++) {
-    Q[a] = Vc[a] = TT(0);
-#pragma unroll
-    for (int b = 0; b < 4; b++) G[a][b] = TT(0);
+  for (int i = 0; i < 3; i++) {
+    uS[i] = rt * ((yl[0][i] + yl[1][i]) + (yl[2][i] + yl[3][i]));
+    aS[i] = rt * ((al[0][i] + al[1][i]) + (al[2][i] + al[3][i])) - A.fb[i];
   }
+  const double pS = rt * ((yl[0][3] + yl[1][3]) + (yl[2][3] + yl[3][3]));
 
-#pragma unroll 1
-  for (int g = 0; g < 4; g++) {
-    double N[4];
+  // sums over the points: of rV2, pa and, for the first three nodes, of the
+  // gradient part of lR (gR) and of up.Nx_a (sU); lN: rd rV2 at node g
+  double vS[3] = {0, 0, 0}, paS = 0.0, gR[3][3], sU[3] = {0, 0, 0}, lN[4][3];
+  // tangent factors (first three nodes): Q = sum tauM uaNx, QU = sum tauM uNx,
+  // UA = sum uaNx, H = the two quadratic sums of S_ab; q2[a][g] = (tauM uaNx_a)
+  // and u2[g][b] = uaNx_b at point g, tMg = tauM at point g
+  const TT rh = TT(rho), rh2 = rh * rh, md = TT(A.fl_amd);
+  TT SC = TT(0), ST = TT(0), Q[3], QU[3], UA[3], H[3][3], q2[3][4], u2[4][3], tMg[4];
 #pragma unroll
-    for (int a = 0; a < 4; a++) N[a] = c_rule.N[g][a];
-    double u[3], ud[3], pr = 0.0;
+  for (int a = 0; a < 3; a++) {
+    Q[a] = QU[a] = UA[a] = TT(0);
 #pragma unroll
-    for (int i = 0; i < 3; i++) {
-      u[i] = N[0] * yl[0][i] + N[1] * yl[1][i] + N[2] * yl[2][i] + N[3] * yl[3][i];
-      ud[i] = -A.fb[i] + N[0] * al[0][i] + N[1] * al[1][i] + N[2] * al[2][i] + N[3] * al[3][i];
+    for (int b = 0; b < 3; b++) {
+      H[a][b] = TT(0);
+      gR[a][b] = 0.0;
     }
+  }
 #pragma unroll
-    for (int a = 0; a < 4; a++) pr += N[a] * yl[a][3];
-    double kU = 0.0;
+  for (int g = 0; g < 4; g++) {
+    double u[3], uN[3], rV[3], up[3], upN[3];
 #pragma unroll
-    for (int j = 0; j < 3; j++)
+    for (int i = 0; i < 3; i++) u[i] = uS[i] + rd * yl[g][i];
+    const double pr = pS + rd * yl[g][3];
 #pragma unroll
-      for (int i = 0; i < 3; i++) kU += u[i] * u[j] * K[i][j];
-    const double tauM = 1.0 / (rho * sqrt(kT + kU + kS));
-    double rV[3], up[3];
+    for (int a = 0; a < 3; a++) uN[a] = u[0] * Nx[0][a] + u[1] * Nx[1][a] + u[2] * Nx[2][a];
+    const double X = kTS + uN[0] * uN[0] + uN[1] * uN[1] + uN[2] * uN[2];
+    const double rX = rsqrt(X);
+    const double tauM = rX * irho, tauC = X * rX * rtrK;
 #pragma unroll
     for (int j = 0; j < 3; j++) {
-      rV[j] = ud[j] + u[0] * ux[0][j] + u[1] * ux[1][j] + u[2] * ux[2][j];
+      rV[j] = (aS[j] + rd * al[g][j]) + u[0] * ux[0][j] + u[1] * ux[1][j] + u[2] * ux[2][j];
       up[j] = -tauM * (rho * rV[j] + px[j]);
     }
-    const double tauC = 1.0 / (tauM * trK);
-    double tauB = 0.0;
 #pragma unroll
-    for (int j = 0; j < 3; j++)
-#pragma unroll
-      for (int i = 0; i < 3; i++) tauB += up[i] * up[j] * K[i][j];
+    for (int a = 0; a < 3; a++) upN[a] = up[0] * Nx[0][a] + up[1] * Nx[1][a] + up[2] * Nx[2][a];
+    double tB2 = upN[0] * upN[0] + upN[1] * upN[1] + upN[2] * upN[2];
     // ISZERO (MATFUN.f:763-780): |x| < eps^2
-    if (fabs(tauB) < 4.930380657631324e-32) tauB = 2.220446049250313e-16;
-    tauB = rho / sqrt(tauB);
-    double ua[3];
-#pragma unroll
-    for (int i = 0; i < 3; i++) ua[i] = u[i] + up[i];
-    const double pa = pr - tauC * divU;
-    double rB[3], rV2[3];
+    if (fabs(tB2) < 4.930380657631324e-32) tB2 = 2.220446049250313e-16;
+    const double tauB = rho * rsqrt(tB2);
+    paS += pr - tauC * divU;
 #pragma unroll
     for (int j = 0; j < 3; j++) {
-      rB[j] = tauB * (up[0] * ux[0][j] + up[1] * ux[1][j] + up[2] * ux[2][j]);
-      rV2[j] = ud[j] + ua[0] * ux[0][j] + ua[1] * ux[1][j] + ua[2] * ux[2][j];
-    }
-    // lR(a,j) += wr N_a rV2_j + w sum_i Nx_i(a) rM(i,j)
+      const double q = up[0] * ux[0][j] + up[1] * ux[1][j] + up[2] * ux[2][j];
+      const double rV2 = rV[j] + q, rB = tauB * q;
+      vS[j] += rV2;
+      lN[g][j] = rV2;
+      // sum_i Nx_i(a) (rB_j up_i - rho up_j ua_i), a < 3
+      const double rup = rho * up[j];
 #pragma unroll
-    for (int j = 0; j < 3; j++) {
-      double rM[3];
-#pragma unroll
-      for (int i = 0; i < 3; i++)
-        rM[i] = mu * es[i][j] - rho * up[j] * ua[i] + rB[j] * up[i] - (i == j ? pa : 0.0);
-#pragma unroll
-      for (int a = 0; a < 4; a++)
-        lR[a][j] += wr * N[a] * rV2[j] + w * (Nx[0][a] * rM[0] + Nx[1][a] * rM[1] + Nx[2][a] * rM[2]);
-    }
-    TT uN[4], upN[4], vN[4];
-#pragma unroll
-    for (int a = 0; a < 4; a++) {
-      const double upNx = up[0] * Nx[0][a] + up[1] * Nx[1][a] + up[2] * Nx[2][a];
-      lR[a][3] += w * (N[a] * divU - upNx);
-      uN[a] = TT(u[0] * Nx[0][a] + u[1] * Nx[1][a] + u[2] * Nx[2][a]);
-      upN[a] = TT(upNx);
-      vN[a] = uN[a] + md * TT(N[a]);
+      for (int a = 0; a < 3; a++) gR[a][j] += rB * upN[a] - rup * (uN[a] + upN[a]);
     }
     const TT tM = TT(tauM), tB = TT(tauB);
     SC += TT(tauC);
     ST += tM;
+    tMg[g] = tM;
+    TT un[3], pn[3];
 #pragma unroll
-    for (int a = 0; a < 4; a++) {
-      const TT uaa = uN[a] + upN[a];
-      Q[a] += tM * uaa;
-      Vc[a] += tM * vN[a];
-      const TT c1 = rh * rh * tM * uaa, c2 = rh * TT(N[a]), c3 = tB * upN[a];
+    for (int a = 0; a < 3; a++) {
+      sU[a] += upN[a];
+      un[a] = TT(uN[a]);
+      pn[a] = TT(upN[a]);
+    }
 #pragma unroll
-      for (int b = 0; b < 4; b++) G[a][b] += c1 * vN[b] + c2 * (uN[b] + upN[b]) + c3 * upN[b];
+    for (int a = 0; a < 3; a++) {
+      const TT ua = un[a] + pn[a], ta = tM * ua;
+      Q[a] += ta;
+      QU[a] += tM * un[a];
+      UA[a] += ua;
+      q2[a][g] = ta;
+      u2[g][a] = ua;
+      const TT c1 = rh2 * ta, c3 = tB * pn[a];
+#pragma unroll
+      for (int b = 0; b < 3; b++) H[a][b] += c1 * un[b] + c3 * pn[b];
     }
   }
-  asm_colour_scatter();
+  // lR(a,j) = wr (rt sum_g rV2_j + rd rV2_j(a)) + w [4 mu es.Nx_a + gR - paS Nx_a]_j,
+  // lR(a,4) = w (Ns_a divU - sum_g up.Nx_a); the bracket sums to zero over a
+  __align__(16) double lR[4][4];
 #pragma unroll
-  for (int a = 0; a < 4; a++)
+  for (int j = 0; j < 3; j++) {
+    double s4 = 0.0;
 #pragma unroll
-    for (int c = 0; c < 4; c++) A.R[(size_t)n4[a] * 4 + c] += lR[a][c];
+    for (int a = 0; a < 3; a++) {
+      const double v =
+          gR[a][j] - paS * Nx[j][a] +
+          4.0 * mu * (Nx[0][a] * es[0][j] + Nx[1][a] * es[1][j] + Nx[2][a] * es[2][j]);
+      s4 -= v;
+      lR[a][j] = w * v;
+    }
+    lR[3][j] = w * s4;
+#pragma unroll
+    for (int a = 0; a < 4; a++) lR[a][j] += wr * (rt * vS[j] + rd * lN[a][j]);
+  }
+  const double wdN = w * c_rule.Ns[0] * divU;
+#pragma unroll
+  for (int a = 0; a < 3; a++) lR[a][3] = wdN - w * sU[a];
+  lR[3][3] = wdN + w * (sU[0] + sU[1] + sU[2]);
 
-  // ---- tangent (TT)
-  const TT mu4 = TT(4.0 * mu), wlt = TT(wl);
+  emit_res<4>(E, &lR[0][0]);
+
+  // ---- tangent (TT), everything scaled by wl
+  const TT wlt = TT(wl), trt = TT(rt), trd = TT(rd), ns = TT(c_rule.Ns[0]);
+  const TT wmu4 = wlt * TT(4.0 * mu), wSC = wlt * SC, wST = wlt * ST, wNs = wlt * ns,
+           wrh = wlt * rh;
   TT Nxa[3][4];
 #pragma unroll
   for (int i = 0; i < 3; i++)
 #pragma unroll
     for (int a = 0; a < 4; a++) Nxa[i][a] = TT(Nx[i][a]);
-  TT *Val = reinterpret_cast<TT *>(A.Val);
+  // wl (G2 + G3 + H)_ab of S_ab: G2 = rho^2 amd sum_g tauM uaNx_a N_b, G3 = rho
+  // sum_g N_a uaNx_b
+  const TT w2 = wlt * rh2 * md;
+  TT S[4][4];
+#pragma unroll
+  for (int a = 0; a < 3; a++)
+#pragma unroll
+    for (int b = 0; b < 4; b++) S[a][b] = w2 * (trt * Q[a] + trd * q2[a][b]);
+#pragma unroll
+  for (int b = 0; b < 4; b++) S[3][b] = -(S[0][b] + S[1][b] + S[2][b]);
+#pragma unroll
+  for (int a = 0; a < 4; a++) {
+    TT s4 = TT(0);
+#pragma unroll
+    for (int b = 0; b < 3; b++) {
+      const TT v = wrh * (trt * UA[b] + trd * u2[a][b]);
+      S[a][b] += v;
+      s4 -= v;
+    }
+    S[a][3] += s4;
+  }
+  {
+    TT h3[4] = {TT(0), TT(0), TT(0), TT(0)};
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+      TT s4 = TT(0);
+#pragma unroll
+      for (int b = 0; b < 3; b++) {
+        const TT v = wlt * H[a][b];
+        S[a][b] += v;
+        s4 -= v;
+        h3[b] -= v;
+      }
+      S[a][3] += s4;
+      h3[3] -= s4;
+    }
+#pragma unroll
+    for (int b = 0; b < 4; b++) S[3][b] += h3[b];
+  }
+  // Q and Vc = sum_g tauM (uNx + amd N) of all four nodes, times wl rho
+  TT Qw[4], Vw[4];
+#pragma unroll
+  for (int a = 0; a < 4; a++) {
+    const TT qa = a < 3 ? Q[a < 3 ? a : 0] : -(Q[0] + Q[1] + Q[2]);
+    const TT qu = a < 3 ? QU[a < 3 ? a : 0] : -(QU[0] + QU[1] + QU[2]);
+    Qw[a] = wrh * qa;
+    Vw[a] = wrh * (qu + md * (trt * ST + trd * tMg[a]));
+  }
   // esNx_i(a) = sum_k es(k,i) Nx_k(a) for the term 4 mu_g esNx_i(a) esNx_j(b)
-  const TT g4 = TT(4.0 * mu_g);
+  const TT g4 = wlt * TT(4.0 * mu_g);
   TT eN[3][4];
 #pragma unroll
   for (int i = 0; i < 3; i++)
 #pragma unroll
     for (int a = 0; a < 4; a++)
       eN[i][a] = NN ? TT(es[0][i] * Nx[0][a] + es[1][i] * Nx[1][a] + es[2][i] * Nx[2][a]) : TT(0);
+  const TT wrM0 = wrh * md;
 #pragma unroll
   for (int a = 0; a < 4; a++) {
-    const int4 m4 = A.map[(size_t)e * 4 + a];
-    const int pos[4] = {m4.x, m4.y, m4.z, m4.w};
+    __align__(16) TT row[64];
+    TT mN[3], cN[3], nN[3];  // 4 mu wl Nx(a), wl sum tauC Nx(a), -wl Ns Nx(a)
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+      mN[i] = wmu4 * Nxa[i][a];
+      cN[i] = wSC * Nxa[i][a];
+      nN[i] = -wNs * Nxa[i][a];
+    }
 #pragma unroll
     for (int b = 0; b < 4; b++) {
       const TT NxNx = Nxa[0][a] * Nxa[0][b] + Nxa[1][a] * Nxa[1][b] + Nxa[2][a] * Nxa[2][b];
-      const TT S = mu4 * NxNx + rh * md * TT(c_rule.M[a][b]) + G[a][b];
-      TT blk[16];
+      const TT Sab = wmu4 * NxNx + (wrM0 * TT(c_rule.M[a][b]) + S[a][b]);
+      TT *v = row + b * 16;
 #pragma unroll
       for (int i = 0; i < 3; i++) {
 #pragma unroll
-        for (int j = 0; j < 3; j++)
-          blk[i * 4 + j] = wlt * (mu4 * Nxa[i][b] * Nxa[j][a] + SC * Nxa[i][a] * Nxa[j][b] +
-                                  (NN ? g4 * eN[i][a] * eN[j][b] : TT(0)) +
-                                  (i == j ? S : TT(0)));
-        blk[i * 4 + 3] = -wlt * (Nxa[i][a] * TT(c_rule.Ns[b]) - rh * Nxa[i][b] * Q[a]);
-        blk[12 + i] = wlt * (TT(c_rule.Ns[a]) * Nxa[i][b] + rh * Nxa[i][a] * Vc[b]);
+        for (int j = 0; j < 3; j++) {
+          v[i * 4 + j] = mN[j] * Nxa[i][b] + (cN[i] * Nxa[j][b] + (i == j ? Sab : TT(0)));
+          if (NN) v[i * 4 + j] += (g4 * eN[i][a]) * eN[j][b];
+        }
+        v[i * 4 + 3] = Qw[a] * Nxa[i][b] + nN[i];
+        v[12 + i] = Vw[b] * Nxa[i][a] + wNs * Nxa[i][b];
       }
-      blk[15] = wlt * ST * NxNx;
-      TT *dst = Val + (size_t)pos[b] * 16;
-#pragma unroll
-      for (int k = 0; k < 16; k++) dst[k] += blk[k];
+      v[15] = wST * NxNx;
     }
+    emit_row<TT, 4>(E, a, row);
   }
 }
 

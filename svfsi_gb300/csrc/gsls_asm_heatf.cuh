@@ -18,7 +18,6 @@ namespace gsls {
 
 template <class VT>
 __global__ void __launch_bounds__(kAsmThreads) k_asm_heatf(AsmArgs A) {
-  asm_colour_start();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= A.nColorEl) return;
   const int e = A.el0 + t;
@@ -40,31 +39,27 @@ __global__ void __launch_bounds__(kAsmThreads) k_asm_heatf(AsmArgs A) {
   // gradients of the first three shape functions, so ks = sum_{a<3} Nx_a
   // Nx_a^T.  The element runs on the FP64 pipe, so its quadratic forms are
   // taken through those gradients, x.ks.x = sum_{a<3} (Nx_a.x)^2 (u.ks.u
-  // and Tx.ks.Tx), and ks:ks from the six distinct entries of the symmetric
-  // ks: the reference's quantities, rounded differently.
-  double k00 = 0, k01 = 0, k02 = 0, k11 = 0, k12 = 0, k22 = 0;
-#pragma unroll
-  for (int a = 0; a < 3; a++) {
-    k00 += Nx[0][a] * Nx[0][a];
-    k01 += Nx[0][a] * Nx[1][a];
-    k02 += Nx[0][a] * Nx[2][a];
-    k11 += Nx[1][a] * Nx[1][a];
-    k12 += Nx[1][a] * Nx[2][a];
-    k22 += Nx[2][a] * Nx[2][a];
-  }
-  const double kS = k00 * k00 + k11 * k11 + k22 * k22 + 2.0 * (k01 * k01 + k02 * k02 + k12 * k12);
+  // and Tx.ks.Tx), ks:ks comes from the geometry table, and what is linear in
+  // Nx_a is minus the sum of the other three at the fourth node: the
+  // reference's quantities, rounded differently.  (Cylinder of 1,225,440
+  // tets, mixed, ten assemblies and solves: 13.6 ms before, 10.9 ms with the
+  // last two and the element buffer.)
+  double kS, trk;
+  load_metric(A, e, kS, trk);
   double Tx[3];
 #pragma unroll
-  for (int i = 0; i < 3; i++) Tx[i] = Nx[i][0] * Ty[0] + Nx[i][1] * Ty[1] + Nx[i][2] * Ty[2] + Nx[i][3] * Ty[3];
+  for (int i = 0; i < 3; i++)
+    Tx[i] = Nx[i][0] * (Ty[0] - Ty[3]) + Nx[i][1] * (Ty[1] - Ty[3]) + Nx[i][2] * (Ty[2] - Ty[3]);
   double NxTx[4];  // Nx_a . Tx (constant on a tet4)
 #pragma unroll
-  for (int a = 0; a < 4; a++) NxTx[a] = Nx[0][a] * Tx[0] + Nx[1][a] * Tx[1] + Nx[2][a] * Tx[2];
+  for (int a = 0; a < 3; a++) NxTx[a] = Nx[0][a] * Tx[0] + Nx[1][a] * Tx[1] + Nx[2][a] * Tx[2];
+  NxTx[3] = -(NxTx[0] + NxTx[1] + NxTx[2]);
   double nTx = NxTx[0] * NxTx[0] + NxTx[1] * NxTx[1] + NxTx[2] * NxTx[2];  // Tx.ks.Tx
   // ISZERO (MATFUN.f:763-780): |x| < eps^2
   if (fabs(nTx) < 4.930380657631324e-32) nTx = 2.220446049250313e-16;
   const double rnTx = 0.5 * rsqrt(nTx);
   const double T1 = A.af * A.gam * A.dt, amd = A.hf_amd, kT = A.hf_kT;
-  VT lK[4][4];
+  __align__(16) VT lK[4][4];
 #pragma unroll
   for (int a = 0; a < 4; a++)
 #pragma unroll
@@ -103,9 +98,9 @@ __global__ void __launch_bounds__(kAsmThreads) k_asm_heatf(AsmArgs A) {
 #pragma unroll
     for (int i = 0; i < 3; i++) u[i] = ys[i] + rd * y[g][i];
     const double Td = Tas + rd * Ta[g];
-    double udNx[4];  // u . Nx_a
+    double udNx[3];  // u . Nx_a
 #pragma unroll
-    for (int a = 0; a < 4; a++) udNx[a] = u[0] * Nx[0][a] + u[1] * Nx[1][a] + u[2] * Nx[2][a];
+    for (int a = 0; a < 3; a++) udNx[a] = u[0] * Nx[0][a] + u[1] * Nx[1][a] + u[2] * Nx[2][a];
     const double kU = udNx[0] * udNx[0] + udNx[1] * udNx[1] + udNx[2] * udNx[2];  // u.ks.u
     const double udTx = u[0] * Tx[0] + u[1] * Tx[1] + u[2] * Tx[2];
     const double r = Td + udTx;
@@ -116,33 +111,39 @@ __global__ void __launch_bounds__(kAsmThreads) k_asm_heatf(AsmArgs A) {
     rsum += r;
     nusum += nu;
 #pragma unroll
-    for (int a = 0; a < 4; a++) lRu[a] += udNx[a] * tr;
-    const VT wn = VT(wl * nu), tv = VT(tauM);
-    VT ta[4], tb[4];
+    for (int a = 0; a < 3; a++) lRu[a] += udNx[a] * tr;
+    const VT tv = VT(tauM);
+    VT ta[4], tb[4], uv[4];
+#pragma unroll
+    for (int a = 0; a < 3; a++) uv[a] = VT(udNx[a]);
+    uv[3] = -(uv[0] + uv[1] + uv[2]);
 #pragma unroll
     for (int a = 0; a < 4; a++) {
-      const VT un = VT(udNx[a]), na = a == g ? nsv : ntv;
+      const VT un = uv[a], na = a == g ? nsv : ntv;
       ta[a] = wlv * (na + tv * un);
       tb[a] = na * amdv + un;
     }
 #pragma unroll
     for (int a = 0; a < 4; a++)
 #pragma unroll
-      for (int b = 0; b < 4; b++) lK[a][b] += wn * NxN[a][b] + ta[a] * tb[b];
+      for (int b = 0; b < 4; b++) lK[a][b] += ta[a] * tb[b];
   }
+  const VT nuv = VT(wl * nusum);
+#pragma unroll
+  for (int a = 0; a < 4; a++)
+#pragma unroll
+    for (int b = 0; b < 4; b++) lK[a][b] += nuv * NxN[a][b];
+  lRu[3] = -(lRu[0] + lRu[1] + lRu[2]);
   double lR[4];
 #pragma unroll
   for (int a = 0; a < 4; a++) lR[a] = rt * rsum + rd * rg[a] + NxTx[a] * nusum + lRu[a];
-  VT *Val = reinterpret_cast<VT *>(A.Val);
-  asm_colour_scatter();
+  // the element's 16 values and 4 residuals are whole vectors of their own
+  double2 *oR = reinterpret_cast<double2 *>(A.lR + (size_t)t * 4);
+  oR[0] = make_double2(w * lR[0], w * lR[1]);
+  oR[1] = make_double2(w * lR[2], w * lR[3]);
+  uint4 *oK = reinterpret_cast<uint4 *>(reinterpret_cast<VT *>(A.lK) + (size_t)t * 16);
 #pragma unroll
-  for (int a = 0; a < 4; a++) {
-    A.R[n4[a]] += w * lR[a];
-    const int4 mp = A.map[(size_t)e * 4 + a];
-    const int pos[4] = {mp.x, mp.y, mp.z, mp.w};
-#pragma unroll
-    for (int b = 0; b < 4; b++) Val[pos[b]] += lK[a][b];
-  }
+  for (int q = 0; q < (int)sizeof(VT); q++) oK[q] = reinterpret_cast<const uint4 *>(&lK[0][0])[q];
 }
 
 }  // namespace gsls

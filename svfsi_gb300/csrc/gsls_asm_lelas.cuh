@@ -18,10 +18,9 @@ namespace gsls {
 
 template <class VT>
 __global__ void __launch_bounds__(kAsmThreads) k_asm_lelas(AsmArgs A) {
-  asm_colour_start();
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= A.nColorEl) return;
-  const int e = A.el0 + t;
+  extern __shared__ __align__(16) unsigned char asm_smem[];
+  const EmitAt E = emit_at(A, asm_smem, emit_bytes<VT, 3>(), sizeof(VT) * 144, 3);
+  const int e = A.el0 + min((int)(blockIdx.x * blockDim.x + threadIdx.x), A.nColorEl - 1);
   const int4 nd = A.ien[e];
   const int n4[4] = {nd.x, nd.y, nd.z, nd.w};
   const int tD = A.tDof, s0 = A.s;
@@ -53,7 +52,7 @@ __global__ void __launch_bounds__(kAsmThreads) k_asm_lelas(AsmArgs A) {
   const double Sxy = mu * ed[3], Syz = mu * ed[4], Sxz = mu * ed[5];
 
   // ---- residual (FP64)
-  asm_colour_scatter();
+  __align__(16) double lR[4][3];
 #pragma unroll
   for (int a = 0; a < 4; a++) {
     double m[3];
@@ -63,10 +62,9 @@ __global__ void __launch_bounds__(kAsmThreads) k_asm_lelas(AsmArgs A) {
 #pragma unroll
       for (int b = 0; b < 4; b++) m[c] += c_rule.M[a][b] * al[b][c];
     }
-    double *R = A.R + (size_t)n4[a] * 3;
-    R[0] += w * rho * m[0] + W * (Nx[0][a] * Sxx + Nx[1][a] * Sxy + Nx[2][a] * Sxz);
-    R[1] += w * rho * m[1] + W * (Nx[0][a] * Sxy + Nx[1][a] * Syy + Nx[2][a] * Syz);
-    R[2] += w * rho * m[2] + W * (Nx[0][a] * Sxz + Nx[1][a] * Syz + Nx[2][a] * Szz);
+    lR[a][0] = w * rho * m[0] + W * (Nx[0][a] * Sxx + Nx[1][a] * Sxy + Nx[2][a] * Sxz);
+    lR[a][1] = w * rho * m[1] + W * (Nx[0][a] * Sxy + Nx[1][a] * Syy + Nx[2][a] * Syz);
+    lR[a][2] = w * rho * m[2] + W * (Nx[0][a] * Sxz + Nx[1][a] * Syz + Nx[2][a] * Szz);
   }
 
   // ---- tangent (VT), symmetric blocks
@@ -77,36 +75,22 @@ __global__ void __launch_bounds__(kAsmThreads) k_asm_lelas(AsmArgs A) {
   for (int i = 0; i < 3; i++)
 #pragma unroll
     for (int a = 0; a < 4; a++) Nxa[i][a] = VT(Nx[i][a]);
-  VT *Val = reinterpret_cast<VT *>(A.Val);
+  emit_res<3>(E, &lR[0][0]);
 #pragma unroll
   for (int a = 0; a < 4; a++) {
-    const int4 m4 = A.map[(size_t)e * 4 + a];
-    const int pos[4] = {m4.x, m4.y, m4.z, m4.w};
+    __align__(16) VT row[36];
 #pragma unroll
-    for (int b = a; b < 4; b++) {
+    for (int b = 0; b < 4; b++) {
       const VT dd = Nxa[0][a] * Nxa[0][b] + Nxa[1][a] * Nxa[1][b] + Nxa[2][a] * Nxa[2][b];
       const VT diag = kM * VT(c_rule.M[a][b]) + kU * dd;
-      VT blk[9];
 #pragma unroll
       for (int r = 0; r < 3; r++)
 #pragma unroll
         for (int c = 0; c < 3; c++)
-          blk[r * 3 + c] = kL * Nxa[r][a] * Nxa[c][b] + kU * Nxa[c][a] * Nxa[r][b] +
-                           ((r == c) ? diag : VT(0));
-      VT *dst = Val + (size_t)pos[b] * 9;
-#pragma unroll
-      for (int k = 0; k < 9; k++) dst[k] += blk[k];
-      if (b > a) {
-        // block (b,a) = block(a,b)^T
-        const int4 mb = A.map[(size_t)e * 4 + b];
-        const int pba = (a == 0) ? mb.x : (a == 1) ? mb.y : (a == 2) ? mb.z : mb.w;
-        VT *dt = Val + (size_t)pba * 9;
-#pragma unroll
-        for (int r = 0; r < 3; r++)
-#pragma unroll
-          for (int c = 0; c < 3; c++) dt[r * 3 + c] += blk[c * 3 + r];
-      }
+          row[b * 9 + r * 3 + c] = kL * Nxa[r][a] * Nxa[c][b] + kU * Nxa[c][a] * Nxa[r][b] +
+                                   ((r == c) ? diag : VT(0));
     }
+    emit_row<VT, 3>(E, a, row);
   }
 }
 

@@ -2,18 +2,21 @@
 // isotropic CEP (CEP.f:136-266), FLUID with VMS stabilisation
 // (FLUID.f:40-1084) and STRUCT with the neo-Hookean + ST91 material
 // (Code/Source/svFSI/STRUCT.f:39-496, MATMODELS.f:41-150,539-564,1588-1647),
-// scattered into block CSR as DOASSEM does (Code/Source/svFSI/LHSA.f:266-298).
+// added into block CSR as DOASSEM does (Code/Source/svFSI/LHSA.f:266-298).
 //
 // GB300 design: the binary search of DOASSEM is replaced by a precomputed
-// element -> CSR position map (16 int32 per tet); the RMW scatter is made
-// race-free and deterministic by a greedy node-conflict colouring (one
-// launch per colour, elements stored in colour order).  One thread owns one
+// element -> CSR position map (16 int32 per tet).  Elements are stored in the
+// order of a greedy node-conflict colouring.  FLUID, inviscid STRUCT, LELAS
+// and HEATF write element matrices to a buffer, from which every CSR block
+// adds its own in that order (gsls_asm_gather.cuh); viscous STRUCT, USTRUCT
+// and the heat element scatter, one launch per colour.  One thread owns one
 // element; the residual is always FP64, the tangent is FP64 (drop-in) or
 // FP32 (mixed precision, with det F, S and P kept in FP64).
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <vector>
 
 #include "gsls_internal.cuh"
@@ -29,6 +32,10 @@ struct gsls_mesh {
   gsls::DevBuf d_x;               // double nNo*3
   gsls::DevBuf d_eparam;          // double per element (colour order)
   gsls::DevBuf d_err;             // int error word
+  // element blocks of each CSR block (gsls_asm_gather.cuh), and the element buffer
+  gsls::DevBuf d_invp, d_inve, d_elK, d_elR;
+  bool inv_ready = false;
+  std::mutex el_mu;               // held while an assembly through the buffer is enqueued
   gsls::DevBuf d_geo;             // per-element Nx (12) and Jacobian, SoA: geo[k * nEl + e]
   bool bad_jac = false;           // a zero or non-finite element Jacobian
   const double *eparam_src = nullptr;
@@ -96,6 +103,7 @@ struct AsmArgs {
   double mu_o, vlam, va, vn;
   double E_s, nu_s;      // USTRUCT elasticity modulus and Poisson ratio (GETTAU)
   int volType;           // USTRUCT volumetric penalty (GVOLPEN)
+  double fl_irho, fl_T1, fl_amd, fl_kT;  // FLUID 1/rho, af gam dt, am / (af gam dt), 4 (ctM/dt)^2
   double hf_amd, hf_kT;  // HEATF am / (af gam dt) and 4 / dt^2, formed once on the host
   const double *fib;     // CEP fibre table (SoA, colour order) or null
   int nFn;               // fibre families in fib
@@ -110,6 +118,8 @@ struct AsmArgs {
   double *R;
   void *Val;
   int *err;
+  void *lK;    // element buffer of the gathered assembly (gsls_asm_gather.cuh)
+  double *lR;
 };
 
 // ---------------------------------------------------------------------------
@@ -117,13 +127,21 @@ struct AsmArgs {
 // function gradients Nx(3,4) and the Jacobian depend on the mesh only, so
 // they are computed once per mesh (adjugate, one division) and read by every
 // assembly as 13 coalesced streams instead of 12 gathered coordinates.
-constexpr int kGeo = 13;  // Nx[i][a] at k = i*4 + a, Jac at k = 12
+// Nx[i][a] at k = i*4 + a, Jac at 12; of the metric tensor ks = sum_{a<3}
+// Nx_a Nx_a^T (GNN, NN.f:1539-1547): ks:ks at 13, tr ks at 14 (27 FP64
+// instructions of every stabilised element otherwise)
+constexpr int kGeo = 15;
 __device__ __forceinline__ double load_geo(const AsmArgs &A, int e, double Nx[3][4]) {
 #pragma unroll
   for (int i = 0; i < 3; i++)
 #pragma unroll
     for (int a = 0; a < 4; a++) Nx[i][a] = __ldg(A.geo + (size_t)(i * 4 + a) * A.nElAll + e);
   return __ldg(A.geo + (size_t)12 * A.nElAll + e);
+}
+
+__device__ __forceinline__ void load_metric(const AsmArgs &A, int e, double &kk, double &trk) {
+  kk = __ldg(A.geo + (size_t)13 * A.nElAll + e);
+  trk = __ldg(A.geo + (size_t)14 * A.nElAll + e);
 }
 
 // Colour launches overlap: each colour kernel lets the next one be
@@ -138,6 +156,7 @@ __device__ __forceinline__ void asm_colour_scatter() { cudaGridDependencySynchro
 
 }  // namespace gsls
 
+#include "gsls_asm_gather.cuh"
 #include "gsls_asm_struct.cuh"
 
 namespace gsls {
@@ -159,6 +178,7 @@ __global__ void k_geo_tet4(int nEl, const int4 *__restrict__ ien, const double *
   const double Jac = adj_det3(xXi, adj);
   if (!(Jac != 0.0) || !isfinite(Jac)) atomicOr(err, 1);
   const double iJ = 1.0 / Jac;
+  double N[3][3];
 #pragma unroll
   for (int i = 0; i < 3; i++) {
     const double n0 = adj[0][i] * iJ, n1 = adj[1][i] * iJ, n2 = adj[2][i] * iJ;
@@ -166,8 +186,22 @@ __global__ void k_geo_tet4(int nEl, const int4 *__restrict__ ien, const double *
     geo[(size_t)(i * 4 + 1) * nEl + e] = n1;
     geo[(size_t)(i * 4 + 2) * nEl + e] = n2;
     geo[(size_t)(i * 4 + 3) * nEl + e] = -(n0 + n1 + n2);
+    N[i][0] = n0;
+    N[i][1] = n1;
+    N[i][2] = n2;
   }
   geo[(size_t)12 * nEl + e] = Jac;
+  double kk = 0.0, trk = 0.0;
+#pragma unroll
+  for (int i = 0; i < 3; i++)
+#pragma unroll
+    for (int j = i; j < 3; j++) {
+      const double k = N[i][0] * N[j][0] + N[i][1] * N[j][1] + N[i][2] * N[j][2];
+      kk += (i == j ? 1.0 : 2.0) * (k * k);
+      if (i == j) trk += k;
+    }
+  geo[(size_t)13 * nEl + e] = kk;
+  geo[(size_t)14 * nEl + e] = trk;
 }
 
 // ---------------------------------------------------------------------------
@@ -453,6 +487,84 @@ static int asm_launch(K kern, int nb, cudaStream_t st, const AsmArgs &A, bool pd
   return GSLS_OK;
 }
 
+// inverse element -> CSR map, on the first gathered assembly of a mesh
+static int inv_prepare(gsls_mesh *m) {
+  if (m->inv_ready) return GSLS_OK;
+  gsls_lhs *lhs = m->lhs;
+  cudaStream_t st = lhs->stream;
+  const int nnz = lhs->nnz, nb = (nnz + kScan - 1) / kScan;
+  const size_t n = (size_t)m->nEl * 16;
+  if (n > 0x7fffffffull) {
+    set_error("assembly: more than 134,217,727 elements");
+    return GSLS_ERR_UNSUPPORTED;
+  }
+  DevBuf cnt, sums;
+  GSLS_TRY(m->d_invp.alloc(sizeof(int) * ((size_t)nnz + 1)));
+  GSLS_TRY(m->d_inve.alloc(sizeof(int) * n));
+  GSLS_TRY(cnt.alloc(sizeof(int) * (size_t)nnz));
+  GSLS_TRY(sums.alloc(sizeof(int) * (size_t)nb));
+  const int *map = m->d_map.as<int>();
+  int *ptr = m->d_invp.as<int>(), *ent = m->d_inve.as<int>();
+  const int g = 8 * num_sms();
+  GSLS_CUDA(cudaMemsetAsync(cnt.p, 0, sizeof(int) * (size_t)nnz, st));
+  k_inv_count<<<g, 256, 0, st>>>(n, map, cnt.as<int>());
+  GSLS_CHECK_LAUNCH();
+  k_scan_sums<<<nb, 256, 0, st>>>(nnz, cnt.as<int>(), sums.as<int>());
+  GSLS_CHECK_LAUNCH();
+  k_scan_top<<<1, 1024, 0, st>>>(nb, sums.as<int>());
+  GSLS_CHECK_LAUNCH();
+  k_scan_fill<<<nb, 256, 0, st>>>(nnz, cnt.as<int>(), sums.as<int>(), ptr, (int)n);
+  GSLS_CHECK_LAUNCH();
+  k_inv_fill<<<g, 256, 0, st>>>(n, map, ptr, cnt.as<int>(), ent);
+  GSLS_CHECK_LAUNCH();
+  k_inv_sort<<<g, 256, 0, st>>>(nnz, ptr, ent);
+  GSLS_CHECK_LAUNCH();
+  GSLS_CUDA(cudaStreamSynchronize(st));  // cnt and sums go out of scope
+  m->inv_ready = true;
+  return GSLS_OK;
+}
+
+// R and Val through the element buffer: kern over all elements (in parts of at
+// most kElemBuf bytes), then the sums; smem: staging bytes per warp
+template <int DOF, class VT, class K>
+static int assemble_gather(gsls_mesh *m, K kern, size_t smem, AsmArgs A, double *R, VT *Val) {
+  std::lock_guard<std::mutex> lk(m->el_mu);
+  GSLS_TRY(inv_prepare(m));
+  constexpr int DD = DOF * DOF;
+  gsls_lhs *lhs = m->lhs;
+  cudaStream_t st = lhs->stream;
+  const size_t per = 16 * DD * sizeof(VT) + 4 * DOF * sizeof(double);
+  int part = (int)std::min<size_t>((size_t)m->nEl, kElemBuf / per);
+  // a device short of memory takes smaller parts
+  while (m->d_elK.alloc(16 * DD * sizeof(VT) * (size_t)part) != GSLS_OK ||
+         m->d_elR.alloc(4 * DOF * sizeof(double) * (size_t)part) != GSLS_OK) {
+    cudaGetLastError();
+    if (part <= 4096) return GSLS_ERR_CUDA;
+    part /= 2;
+  }
+  A.lK = m->d_elK.p;
+  A.lR = m->d_elR.as<double>();
+  const size_t sm = smem * (kAsmThreads / 32);
+  if (sm > 48 * 1024)
+    GSLS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+  const int *ptr = m->d_invp.as<int>(), *ent = m->d_inve.as<int>();
+  for (int e0 = 0; e0 < m->nEl; e0 += part) {
+    const int ne = std::min(part, m->nEl - e0);
+    A.el0 = e0;
+    A.nColorEl = ne;
+    kern<<<(ne + kAsmThreads - 1) / kAsmThreads, kAsmThreads, sm, st>>>(A);
+    GSLS_CHECK_LAUNCH();
+    const size_t n = (size_t)lhs->nnz * DD;
+    k_gather_val<DD, VT><<<(unsigned)std::min<size_t>((n + 255) / 256, 1u << 20), 256, 0, st>>>(
+        n, ptr, ent, m->d_elK.as<VT>(), e0, e0 + ne, e0 == 0, Val);
+    GSLS_CHECK_LAUNCH();
+    k_gather_res<DOF><<<(lhs->nNo * DOF + 255) / 256, 256, 0, st>>>(
+        lhs->nNo, lhs->d_diagPtr.as<int>(), ptr, ent, A.lR, e0, e0 + ne, e0 == 0, R);
+    GSLS_CHECK_LAUNCH();
+  }
+  return GSLS_OK;
+}
+
 // ---------------------------------------------------------------------------
 static int launch_assembly(gsls_mesh *m, const gsls_eq_params *p, const double *Ag,
                            const double *Yg, const double *Dg, double *R, void *Val,
@@ -504,6 +616,10 @@ static int launch_assembly(gsls_mesh *m, const gsls_eq_params *p, const double *
   A.E_s = p->elM;
   A.nu_s = p->nu;
   A.volType = p->volType;
+  A.fl_irho = 1.0 / p->rho;
+  A.fl_T1 = p->af * p->gam * p->dt;
+  A.fl_amd = p->am / A.fl_T1;
+  A.fl_kT = 4.0 * (p->ctM / p->dt) * (p->ctM / p->dt);
   A.hf_amd = p->am / (p->af * p->gam * p->dt);
   A.hf_kT = 4.0 / (p->dt * p->dt);
   A.nFn = (p->phys == GSLS_PHYS_CEP) ? m->nFn : 0;  // only CEP reads the mesh's fibres
@@ -575,6 +691,33 @@ static int launch_assembly(gsls_mesh *m, const gsls_eq_params *p, const double *
     }
     return GSLS_OK;
   }
+#define GSLS_GATHER(DOF, K32, K64)                                                             \
+  (mixed ? assemble_gather<DOF, float>(m, K32, DOF == 1 ? 0 : emit_bytes<float, DOF>(), A, R,  \
+                                       static_cast<float *>(Val))                              \
+         : assemble_gather<DOF, double>(m, K64, DOF == 1 ? 0 : emit_bytes<double, DOF>(), A,   \
+                                        R, static_cast<double *>(Val)))
+  if (p->phys == GSLS_PHYS_STRUCT && p->visc == 0.0) {
+    if (dof != 3 || p->s + 3 > p->tDof || !Dg) return GSLS_ERR_ARG;
+    return GSLS_GATHER(3, k_asm_struct_nh<float>, k_asm_struct_nh<double>);
+  }
+  if (p->phys == GSLS_PHYS_FLUID) {
+    if (dof != 4 || p->s + 4 > p->tDof || !(p->rho > 0.0) || !(p->dt > 0.0)) return GSLS_ERR_ARG;
+    if (p->viscType != GSLS_VISC_CONST)
+      return GSLS_GATHER(4, (k_asm_fluid<float, true>), (k_asm_fluid<double, true>));
+    return GSLS_GATHER(4, (k_asm_fluid<float, false>), (k_asm_fluid<double, false>));
+  }
+  if (p->phys == GSLS_PHYS_HEATF) {
+    if (dof != 1 || p->tDof < 4 || p->s < 3 || p->s >= p->tDof || !(p->dt > 0.0))
+      return GSLS_ERR_ARG;
+    return GSLS_GATHER(1, k_asm_heatf<float>, k_asm_heatf<double>);
+  }
+  if (p->phys == GSLS_PHYS_LELAS) {
+    if (dof != 3 || p->s + 3 > p->tDof || !Dg || !(p->elM > 0.0) || !(p->nu > -1.0) ||
+        !(p->nu < 0.5) || !(p->dt > 0.0))
+      return GSLS_ERR_ARG;
+    return GSLS_GATHER(3, k_asm_lelas<float>, k_asm_lelas<double>);
+  }
+#undef GSLS_GATHER
   GSLS_CUDA(cudaMemsetAsync(R, 0, sizeof(double) * (size_t)lhs->nNo * dof, st));
   GSLS_CUDA(cudaMemsetAsync(Val, 0, vbytes, st));
   if (p->phys == GSLS_PHYS_USTRUCT)
@@ -598,35 +741,11 @@ static int launch_assembly(gsls_mesh *m, const gsls_eq_params *p, const double *
         GSLS_TRY(asm_launch(k_asm_struct<float>, nb, st, A, pdl));
       else
         GSLS_TRY(asm_launch(k_asm_struct<double>, nb, st, A, pdl));
-    } else if (p->phys == GSLS_PHYS_FLUID) {
-      if (dof != 4 || p->s + 4 > p->tDof || !(p->rho > 0.0) || !(p->dt > 0.0)) return GSLS_ERR_ARG;
-      const bool nn = (p->viscType != GSLS_VISC_CONST);
-      if (mixed)
-        GSLS_TRY(asm_launch(nn ? k_asm_fluid<float, true> : k_asm_fluid<float, false>, nb, st, A,
-                            pdl));
-      else
-        GSLS_TRY(asm_launch(nn ? k_asm_fluid<double, true> : k_asm_fluid<double, false>, nb, st,
-                            A, pdl));
-    } else if (p->phys == GSLS_PHYS_HEATF) {
-      if (dof != 1 || p->tDof < 4 || p->s < 3 || p->s >= p->tDof || !(p->dt > 0.0))
-        return GSLS_ERR_ARG;
-      if (mixed)
-        GSLS_TRY(asm_launch(k_asm_heatf<float>, nb, st, A, pdl));
-      else
-        GSLS_TRY(asm_launch(k_asm_heatf<double>, nb, st, A, pdl));
     } else if (p->phys == GSLS_PHYS_USTRUCT) {
       if (mixed)
         k_asm_ustruct<float><<<nb, kAsmThreads, 0, st>>>(A, Kd);
       else
         k_asm_ustruct<double><<<nb, kAsmThreads, 0, st>>>(A, Kd);
-    } else if (p->phys == GSLS_PHYS_LELAS) {
-      if (dof != 3 || p->s + 3 > p->tDof || !Dg || !(p->elM > 0.0) || !(p->nu > -1.0) ||
-          !(p->nu < 0.5) || !(p->dt > 0.0))
-        return GSLS_ERR_ARG;
-      if (mixed)
-        GSLS_TRY(asm_launch(k_asm_lelas<float>, nb, st, A, pdl));
-      else
-        GSLS_TRY(asm_launch(k_asm_lelas<double>, nb, st, A, pdl));
     } else {
       set_error("assembly: physics not built in this version of the library");
       return GSLS_ERR_UNSUPPORTED;
