@@ -10,12 +10,14 @@
 // (6.3 GB of DRAM traffic for a 188 MB matrix on the neo-Hookean beam).  The
 // buffer is written and read once, in whole sectors.  The elements are stored
 // in colour order, so a block's sum takes the colours' order: the same sum.
-// A buffer above kElemBuf is filled and added in parts.
+// A buffer above kElemBuf is filled and added in parts; the map is one list per
+// window of kInvEl elements, so that its entries fit in 31 bits.
 #pragma once
 
 namespace gsls {
 
 constexpr size_t kElemBuf = (size_t)4 << 30;
+constexpr int kInvEl = 1 << 26;
 
 // One warp's rows of N values per lane, staged in shared memory so that the
 // rows leave in whole 16-byte vectors, each row contiguous.  PAD: an odd

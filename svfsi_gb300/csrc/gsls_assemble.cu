@@ -16,6 +16,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <memory>
 #include <mutex>
 #include <vector>
 
@@ -32,8 +33,13 @@ struct gsls_mesh {
   gsls::DevBuf d_x;               // double nNo*3
   gsls::DevBuf d_eparam;          // double per element (colour order)
   gsls::DevBuf d_err;             // int error word
-  // element blocks of each CSR block (gsls_asm_gather.cuh), and the element buffer
-  gsls::DevBuf d_invp, d_inve, d_elK, d_elR;
+  // element blocks of each CSR block (gsls_asm_gather.cuh), one map per window
+  // of kInvEl elements, and the element buffer
+  struct Inverse {
+    gsls::DevBuf ptr, ent;
+  };
+  std::vector<std::unique_ptr<Inverse>> inv;
+  gsls::DevBuf d_elK, d_elR;
   bool inv_ready = false;
   std::mutex el_mu;               // held while an assembly through the buffer is enqueued
   gsls::DevBuf d_geo;             // per-element Nx (12) and Jacobian, SoA: geo[k * nEl + e]
@@ -492,33 +498,34 @@ static int inv_prepare(gsls_mesh *m) {
   if (m->inv_ready) return GSLS_OK;
   gsls_lhs *lhs = m->lhs;
   cudaStream_t st = lhs->stream;
-  const int nnz = lhs->nnz, nb = (nnz + kScan - 1) / kScan;
-  const size_t n = (size_t)m->nEl * 16;
-  if (n > 0x7fffffffull) {
-    set_error("assembly: more than 134,217,727 elements");
-    return GSLS_ERR_UNSUPPORTED;
-  }
+  const int nnz = lhs->nnz, nb = (nnz + kScan - 1) / kScan, g = 8 * num_sms();
   DevBuf cnt, sums;
-  GSLS_TRY(m->d_invp.alloc(sizeof(int) * ((size_t)nnz + 1)));
-  GSLS_TRY(m->d_inve.alloc(sizeof(int) * n));
   GSLS_TRY(cnt.alloc(sizeof(int) * (size_t)nnz));
   GSLS_TRY(sums.alloc(sizeof(int) * (size_t)nb));
-  const int *map = m->d_map.as<int>();
-  int *ptr = m->d_invp.as<int>(), *ent = m->d_inve.as<int>();
-  const int g = 8 * num_sms();
-  GSLS_CUDA(cudaMemsetAsync(cnt.p, 0, sizeof(int) * (size_t)nnz, st));
-  k_inv_count<<<g, 256, 0, st>>>(n, map, cnt.as<int>());
-  GSLS_CHECK_LAUNCH();
-  k_scan_sums<<<nb, 256, 0, st>>>(nnz, cnt.as<int>(), sums.as<int>());
-  GSLS_CHECK_LAUNCH();
-  k_scan_top<<<1, 1024, 0, st>>>(nb, sums.as<int>());
-  GSLS_CHECK_LAUNCH();
-  k_scan_fill<<<nb, 256, 0, st>>>(nnz, cnt.as<int>(), sums.as<int>(), ptr, (int)n);
-  GSLS_CHECK_LAUNCH();
-  k_inv_fill<<<g, 256, 0, st>>>(n, map, ptr, cnt.as<int>(), ent);
-  GSLS_CHECK_LAUNCH();
-  k_inv_sort<<<g, 256, 0, st>>>(nnz, ptr, ent);
-  GSLS_CHECK_LAUNCH();
+  const size_t nw = ((size_t)m->nEl + kInvEl - 1) / kInvEl;
+  m->inv.clear();
+  for (size_t w = 0; w < nw; w++) {
+    m->inv.emplace_back(new gsls_mesh::Inverse);
+    gsls_mesh::Inverse &v = *m->inv.back();
+    const size_t n = 16 * std::min<size_t>(kInvEl, (size_t)m->nEl - w * kInvEl);
+    GSLS_TRY(v.ptr.alloc(sizeof(int) * ((size_t)nnz + 1)));
+    GSLS_TRY(v.ent.alloc(sizeof(int) * n));
+    const int *map = m->d_map.as<int>() + 16 * kInvEl * w;
+    int *ptr = v.ptr.as<int>(), *ent = v.ent.as<int>();
+    GSLS_CUDA(cudaMemsetAsync(cnt.p, 0, sizeof(int) * (size_t)nnz, st));
+    k_inv_count<<<g, 256, 0, st>>>(n, map, cnt.as<int>());
+    GSLS_CHECK_LAUNCH();
+    k_scan_sums<<<nb, 256, 0, st>>>(nnz, cnt.as<int>(), sums.as<int>());
+    GSLS_CHECK_LAUNCH();
+    k_scan_top<<<1, 1024, 0, st>>>(nb, sums.as<int>());
+    GSLS_CHECK_LAUNCH();
+    k_scan_fill<<<nb, 256, 0, st>>>(nnz, cnt.as<int>(), sums.as<int>(), ptr, (int)n);
+    GSLS_CHECK_LAUNCH();
+    k_inv_fill<<<g, 256, 0, st>>>(n, map, ptr, cnt.as<int>(), ent);
+    GSLS_CHECK_LAUNCH();
+    k_inv_sort<<<g, 256, 0, st>>>(nnz, ptr, ent);
+    GSLS_CHECK_LAUNCH();
+  }
   GSLS_CUDA(cudaStreamSynchronize(st));  // cnt and sums go out of scope
   m->inv_ready = true;
   return GSLS_OK;
@@ -547,19 +554,21 @@ static int assemble_gather(gsls_mesh *m, K kern, size_t smem, AsmArgs A, double 
   const size_t sm = smem * (kAsmThreads / 32);
   if (sm > 48 * 1024)
     GSLS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-  const int *ptr = m->d_invp.as<int>(), *ent = m->d_inve.as<int>();
-  for (int e0 = 0; e0 < m->nEl; e0 += part) {
-    const int ne = std::min(part, m->nEl - e0);
+  for (int e0 = 0, ne = 0; e0 < m->nEl; e0 += ne) {
+    // elements of this part, all in one window of the inverse map
+    const int w = e0 / kInvEl, f = e0 - w * kInvEl;
+    ne = std::min(std::min(part, m->nEl - e0), kInvEl - f);
+    const int *ptr = m->inv[w]->ptr.as<int>(), *ent = m->inv[w]->ent.as<int>();
     A.el0 = e0;
     A.nColorEl = ne;
     kern<<<(ne + kAsmThreads - 1) / kAsmThreads, kAsmThreads, sm, st>>>(A);
     GSLS_CHECK_LAUNCH();
     const size_t n = (size_t)lhs->nnz * DD;
     k_gather_val<DD, VT><<<(unsigned)std::min<size_t>((n + 255) / 256, 1u << 20), 256, 0, st>>>(
-        n, ptr, ent, m->d_elK.as<VT>(), e0, e0 + ne, e0 == 0, Val);
+        n, ptr, ent, m->d_elK.as<VT>(), f, f + ne, e0 == 0, Val);
     GSLS_CHECK_LAUNCH();
     k_gather_res<DOF><<<(lhs->nNo * DOF + 255) / 256, 256, 0, st>>>(
-        lhs->nNo, lhs->d_diagPtr.as<int>(), ptr, ent, A.lR, e0, e0 + ne, e0 == 0, R);
+        lhs->nNo, lhs->d_diagPtr.as<int>(), ptr, ent, A.lR, f, f + ne, e0 == 0, R);
     GSLS_CHECK_LAUNCH();
   }
   return GSLS_OK;

@@ -1,6 +1,7 @@
 """Assembly through the element buffer, SpMV lane groups and the GMRES column
 rotation at the sizes where their work splits: meshes of one element, fewer
-elements than a warp, one more than a block of 128; SpMV systems on both
+elements than a warp, one more than a block of 128, and one whose FP64 element
+matrices (4.4 GB) take the buffer twice; SpMV systems on both
 sides of the lane-group rule; Krylov spaces on both sides of the 32 rotations
 that one turn takes.
 
@@ -11,6 +12,7 @@ or 40 of 6e-8 (FP32 tangents, 7e-5).  SpMV: sums of at most 60 products, 60 x 1.
 on a system with condition number < 10.
 """
 import ctypes as C
+import dataclasses
 
 import numpy as np
 import pytest
@@ -21,6 +23,11 @@ pytestmark = pytest.mark.gpu
 
 
 def _problem(phys, nx, ny, nz):
+    if phys == "fluid" and nx:
+        x, ien = meshgen.kuhn_box(nx, ny, nz, 4.0, 1.0, 1.0)
+        rp, cp = meshgen.csr_from_ien(x.shape[0], ien)
+        return dataclasses.replace(_problem("fluid", 0, 0, 0), x=x, ien=ien, rowPtr=rp, colPtr=cp,
+                                   dirichlet=[], traction=[], neumann=[], Y0=None)
     build = {"struct": problems.struct_beam, "lelas": problems.lelas_beam}.get(phys)
     if build:
         return build(nx, ny, nz)
@@ -32,7 +39,8 @@ def _problem(phys, nx, ny, nz):
 @pytest.mark.parametrize("phys,n", [("struct", (1, 1, 1)), ("struct", (3, 1, 1)),
                                     ("struct", (11, 1, 2)), ("struct", (7, 3, 3)),
                                     ("lelas", (1, 1, 1)), ("lelas", (5, 2, 2)),
-                                    ("fluid", None), ("heatf", None)])
+                                    ("fluid", None), ("heatf", None),
+                                    ("fluid", (176, 44, 44))])
 def test_gathered_assembly_matches_oracle(gsls, orc, phys, n, mixed):
     torch = pytest.importorskip("torch")
     p = _problem(phys, *(n or (0, 0, 0)))
