@@ -165,35 +165,59 @@ __global__ void k_inv_sort(int nnz, const int *__restrict__ ptr, int *__restrict
   }
 }
 
-// Val[p] = sum of the element blocks e0 <= e < e1 of its list (added to Val
-// unless first), one thread per value, four loads in flight
+// Values per thread.  The index work is done once per thread: with one value
+// each, 3x3 blocks in FP32 took 270 M warp instructions (342 us for 1,022,208
+// tets), and a row each is faster (neo-Hookean beam, FP32: assembly 1.85 -> 1.67
+// ms).  Of 4x4 blocks in FP64, which are whole sectors, two values each are
+// slower (VMS fluid, 371,520 tets: 1.38 -> 1.49 ms; 48 registers and half the
+// loads in flight).
 template <int DD, class VT>
+constexpr int gather_width() {
+  return DD == 9 && sizeof(VT) == 4 ? 3 : 1;
+}
+// Val[p] = sum of the element blocks e0 <= e < e1 of its list (added to Val
+// unless first), V values per thread, four blocks in flight; PART: the list may
+// hold elements outside e0 .. e1.  Bound by the sectors of the scattered blocks.
+template <int DD, class VT, bool PART>
 __global__ void __launch_bounds__(256) k_gather_val(size_t n, const int *__restrict__ ptr,
                                                     const int *__restrict__ ent,
                                                     const VT *__restrict__ lK, int e0, int e1,
                                                     int first, VT *__restrict__ Val) {
+  constexpr int V = gather_width<DD, VT>(), T = DD / V;
   for (size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x; k < n;
        k += (size_t)gridDim.x * blockDim.x) {
-    const size_t p = k / DD;
-    const int c = (int)(k - p * DD);
+    const size_t p = k / T;
+    const int c = (int)(k - p * T) * V;
     const int b = __ldg(ptr + p), e = __ldg(ptr + p + 1);
-    VT s = first ? VT(0) : Val[k];
+    VT *__restrict__ out = Val + p * DD + c;
+    VT s[V];
+#pragma unroll
+    for (int q = 0; q < V; q++) s[q] = first ? VT(0) : out[q];
+    const VT *__restrict__ src = lK + c - (size_t)e0 * 16 * DD;
     for (int i = b; i < e; i += 4) {
       int id[4];
-      VT v[4];
+      VT v[4][V];
 #pragma unroll
       for (int u = 0; u < 4; u++) {
         id[u] = i + u < e ? __ldg(ent + i + u) : -1;
-        if (id[u] >= 0 && ((id[u] >> 4) < e0 || (id[u] >> 4) >= e1)) id[u] = -1;
+        if (PART && id[u] >= 0 && ((id[u] >> 4) < e0 || (id[u] >> 4) >= e1)) id[u] = -1;
+      }
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        if (id[u] >= 0) {
+          const VT *__restrict__ w = src + (size_t)id[u] * DD;
+#pragma unroll
+          for (int q = 0; q < V; q++) v[u][q] = __ldcs(w + q);
+        }
       }
 #pragma unroll
       for (int u = 0; u < 4; u++)
-        v[u] = id[u] >= 0 ? __ldcs(lK + ((size_t)id[u] - (size_t)e0 * 16) * DD + c) : VT(0);
+        if (id[u] >= 0)
 #pragma unroll
-      for (int u = 0; u < 4; u++)
-        if (id[u] >= 0) s += v[u];
+          for (int q = 0; q < V; q++) s[q] += v[u][q];
     }
-    Val[k] = s;
+#pragma unroll
+    for (int q = 0; q < V; q++) out[q] = s[q];
   }
 }
 // R of a node from the list of its diagonal block, whose entries are (e, a, a)

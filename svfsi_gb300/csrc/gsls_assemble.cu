@@ -563,9 +563,14 @@ static int assemble_gather(gsls_mesh *m, K kern, size_t smem, AsmArgs A, double 
     A.nColorEl = ne;
     kern<<<(ne + kAsmThreads - 1) / kAsmThreads, kAsmThreads, sm, st>>>(A);
     GSLS_CHECK_LAUNCH();
-    const size_t n = (size_t)lhs->nnz * DD;
-    k_gather_val<DD, VT><<<(unsigned)std::min<size_t>((n + 255) / 256, 1u << 20), 256, 0, st>>>(
-        n, ptr, ent, m->d_elK.as<VT>(), f, f + ne, e0 == 0, Val);
+    const size_t n = (size_t)lhs->nnz * (DD / gather_width<DD, VT>());
+    const unsigned gv = (unsigned)std::min<size_t>((n + 255) / 256, 1u << 20);
+    if (ne == m->nEl)
+      k_gather_val<DD, VT, false><<<gv, 256, 0, st>>>(n, ptr, ent, m->d_elK.as<VT>(), f, f + ne,
+                                                      1, Val);
+    else
+      k_gather_val<DD, VT, true><<<gv, 256, 0, st>>>(n, ptr, ent, m->d_elK.as<VT>(), f, f + ne,
+                                                     e0 == 0, Val);
     GSLS_CHECK_LAUNCH();
     k_gather_res<DOF><<<(lhs->nNo * DOF + 255) / 256, 256, 0, st>>>(
         lhs->nNo, lhs->d_diagPtr.as<int>(), ptr, ent, A.lR, f, f + ne, e0 == 0, R);

@@ -55,16 +55,18 @@ def test_gathered_assembly_matches_oracle(gsls, orc, phys, n, mixed):
     mesh = fsils.Mesh(lhs, p.ien, p.x)
     t = [torch.tensor(a, dtype=torch.float64, device="cuda") for a in (A, Y, D)]
     dR = torch.full((p.nNo * p.dof,), 7.0, dtype=torch.float64, device="cuda")
-    dV = torch.full((p.nnz * p.dof ** 2,), 7.0, device="cuda",
+    nv = p.nnz * p.dof ** 2
+    dV = torch.full((nv + 1,), 7.0, device="cuda",
                     dtype=torch.float32 if mixed else torch.float64)
     prm = p.eq_params()
     torch.cuda.synchronize()
-    for _ in range(2):
+    for o in (0, 1):  # the second matrix starts off a 16-byte boundary
+        dst = dV[o:o + nv]
         _lib.check(gsls.gsls_assemble_dev(mesh.h, C.byref(prm), *(C.c_void_p(q.data_ptr()) for q in t),
-                                          C.c_void_p(dR.data_ptr()), C.c_void_p(dV.data_ptr()),
+                                          C.c_void_p(dR.data_ptr()), C.c_void_p(dst.data_ptr()),
                                           fsils.PREC_MIXED if mixed else fsils.PREC_FP64))
         torch.cuda.synchronize()
-        R, V = dR.cpu().numpy(), dV.cpu().numpy().astype(np.float64)
+        R, V = dR.cpu().numpy(), dst.cpu().numpy().astype(np.float64)
         assert np.abs(R - R0.ravel()).max() <= 1e-12 * np.abs(R0).max()
         assert np.abs(V - V0.ravel()).max() <= (7e-5 if mixed else 1e-12) * np.abs(V0).max()
     mesh.free()
