@@ -1143,15 +1143,17 @@ int solve_dev(gsls_lhs *lhs, gsls_ls *ls, int dof, double *dRi, void *dVal, int 
 #undef GSLS_SOLVE_CASE
 }
 
-// LN groups of D lanes per row, the most (of 1, 2, 4; 1, 2 for D = 3) that half
-// the resident warps cover in one pass; scalar rows at least 2, whose lanes
-// would otherwise walk 32 rows apart (20^3 cube, 9,261 scalar rows: 13.9 ->
-// 12.8 us a call with 4, most of it launch and synchronisation)
+// LN groups of D lanes per row, the most (of 1, 2, 4; 1, 2 for D = 3 and for
+// FP32 values, whose sums keep their order: spmv_row_comp) that half the
+// resident warps cover in one pass; scalar rows at least 2, whose lanes would
+// otherwise walk 32 rows apart (20^3 cube, 9,261 scalar rows: 13.9 -> 12.8 us a
+// call with 4, most of it launch and synchronisation)
 template <int D, int VD, class VT, class XT>
 static int spmv_ln(gsls_lhs *lhs, const VT *Val, const XT *x, double *y, bool after) {
   const int nNo = lhs->nNo;
   const long long half = 32LL * num_sms();
-  int LN = D == 3 ? 2 : 4;
+  constexpr int kMax = D == 3 || sizeof(VT) == 4 ? 2 : 4;
+  int LN = kMax;
   while (LN > (D == 1 ? 2 : 1) && (long long)nNo * LN * D > half * 32) LN /= 2;
   const long long rows = LN == 4 ? 32 / D / 4 : LN == 2 ? 32 / D / 2 : 32 / D;
   const long long warps = ((long long)nNo + rows - 1) / rows;
@@ -1165,7 +1167,7 @@ static int spmv_ln(gsls_lhs *lhs, const VT *Val, const XT *x, double *y, bool af
   cfg.attrs = at;
   cfg.numAttrs = 1;
   const int *rp = lhs->d_rowPtr.as<int>(), *cp = lhs->d_colPtr.as<int>();
-  if constexpr (D != 3)
+  if constexpr (kMax == 4)
     if (LN == 4)
       GSLS_CUDA(cudaLaunchKernelEx(&cfg, k_spmv_ln<D, 4, VD, VT, XT, double>, nNo, rp, cp, Val, x, y));
   if (LN == 2)

@@ -89,13 +89,19 @@ struct GatherDir {
 };
 
 // y_r of block row i for lane component r (LN > 1: of its blocks part, part +
-// LN, ...)
+// LN, ...).  One lane adds its blocks in two chains, of even and of odd place
+// in the row.  With FP32 values and LN = 2 each of the two lanes carries one of
+// the row's chains, so the sum has the bits of LN = 1: an FP32 sum in another
+// order differs by 1e-7, far above the FP64 y that a caller gets.  LN = 4 has
+// no such order and is for FP64 values.
 template <int D, class VT, class AT, int LN = 1, class G>
 __device__ __forceinline__ AT spmv_row_comp(int i, int r, const int *__restrict__ rowPtr,
                                             const int *__restrict__ colPtr,
                                             const VT *__restrict__ Val, const G &g,
                                             int part = 0) {
   constexpr int DD = D * D;
+  static_assert(sizeof(AT) == 8 || LN <= 2, "FP32 sums keep their order");
+  constexpr bool kOneChain = sizeof(AT) == 4 && LN == 2;
   const int rs = __ldg(rowPtr + i), re = __ldg(rowPtr + i + 1);
   const VT *__restrict__ v = Val + (size_t)rs * DD + r * D;
   AT acc0 = AT(0), acc1 = AT(0);
@@ -121,7 +127,7 @@ __device__ __forceinline__ AT spmv_row_comp(int i, int r, const int *__restrict_
     for (int u = 0; u < U; u++)
 #pragma unroll
       for (int c = 0; c < D; c++) {
-        if (u & 1)
+        if ((u & 1) && !kOneChain)
           acc1 = fma(a[u][c], xg[u][c], acc1);
         else
           acc0 = fma(a[u][c], xg[u][c], acc0);
@@ -150,7 +156,8 @@ __global__ void __launch_bounds__(256) k_spmv(int nNo, const int *__restrict__ r
 }
 
 // y = K x with LN groups of D lanes per block row (blocks strided by LN, four
-// of each group's loads in flight); the groups' sums are added by shuffles.
+// of each group's loads in flight); the groups' sums are added by shuffles
+// (spmv_row_comp: FP32 sums keep their bits).
 // A small system has too few rows to fill the SMs with a group each, and a
 // row is then a chain of ~4 rounds of dependent loads instead of one or two.
 template <int D, int LN, int VD, class VT, class XT, class YT>
