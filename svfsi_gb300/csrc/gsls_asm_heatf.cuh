@@ -18,6 +18,7 @@ namespace gsls {
 
 template <class VT>
 __global__ void __launch_bounds__(kAsmThreads) k_asm_heatf(AsmArgs A) {
+  constexpr bool f32 = sizeof(VT) == 4;
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= A.nColorEl) return;
   const int e = A.el0 + t;
@@ -112,11 +113,16 @@ __global__ void __launch_bounds__(kAsmThreads) k_asm_heatf(AsmArgs A) {
     nusum += nu;
 #pragma unroll
     for (int a = 0; a < 3; a++) lRu[a] += udNx[a] * tr;
-    const VT tv = VT(tauM);
+    // FP32 tangents: the fourth node's u.Nx is formed in FP64 and rounded as the
+    // others are (minus the sum of three rounded values has their error, which
+    // on a flat element is many times a small gradient), and the diffusive
+    // part is added point by point, in the order of the FP32 sum
+    const VT tv = VT(tauM), wn = VT(wl * nu);
     VT ta[4], tb[4], uv[4];
 #pragma unroll
     for (int a = 0; a < 3; a++) uv[a] = VT(udNx[a]);
-    uv[3] = -(uv[0] + uv[1] + uv[2]);
+    uv[3] = f32 ? VT(u[0] * Nx[0][3] + u[1] * Nx[1][3] + u[2] * Nx[2][3])
+                : -(uv[0] + uv[1] + uv[2]);
 #pragma unroll
     for (int a = 0; a < 4; a++) {
       const VT un = uv[a], na = a == g ? nsv : ntv;
@@ -126,13 +132,19 @@ __global__ void __launch_bounds__(kAsmThreads) k_asm_heatf(AsmArgs A) {
 #pragma unroll
     for (int a = 0; a < 4; a++)
 #pragma unroll
-      for (int b = 0; b < 4; b++) lK[a][b] += ta[a] * tb[b];
+      for (int b = 0; b < 4; b++)
+        if (f32)
+          lK[a][b] += wn * NxN[a][b] + ta[a] * tb[b];
+        else
+          lK[a][b] += ta[a] * tb[b];
   }
-  const VT nuv = VT(wl * nusum);
+  if (!f32) {
+    const VT nuv = VT(wl * nusum);
 #pragma unroll
-  for (int a = 0; a < 4; a++)
+    for (int a = 0; a < 4; a++)
 #pragma unroll
-    for (int b = 0; b < 4; b++) lK[a][b] += nuv * NxN[a][b];
+      for (int b = 0; b < 4; b++) lK[a][b] += nuv * NxN[a][b];
+  }
   lRu[3] = -(lRu[0] + lRu[1] + lRu[2]);
   double lR[4];
 #pragma unroll
