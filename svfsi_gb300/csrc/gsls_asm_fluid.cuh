@@ -29,10 +29,14 @@
 //  * N_a(g) = t + (s - t) d_ag: point values are t sum_a y_a + (s - t) y_g, and
 //    sums over the points of N_a(g) f_g are t sum_g f_g + (s - t) f_a;
 //  * sum_a Nx_a = 0: every quantity f.Nx_a, and every sum of them, is formed
-//    for three nodes and is minus their sum at the fourth;
+//    for three nodes and is minus their sum at the fourth (not in an FP32
+//    tangent, see below);
 //  * x.K.x = sum_{a<3} (x.Nx_a)^2 for the metric tensor K = sum_{a<3} Nx_a Nx_a^T;
 //  * div-free scalars: 1/rho, amd, 4 (ctM/dt)^2 come from the host, tauM,
 //    tauC and tauB from one rsqrt each instead of roots and divisions.
+// An FP32 tangent forms u.Nx and up.Nx of all four nodes in FP64 and carries
+// all 4 x 4 sums: minus the sum of three rounded values has the error of the
+// largest of them, on a flat element many times the fourth.
 // FP64 assembly of the h = 0.04 cylinder (371,520 tets): 2.87 ms before, 1.38
 // ms with these and the element buffer (3.3 ms with these and the colour
 // scatter).
@@ -141,20 +145,22 @@ __global__ void __launch_bounds__(kAsmThreads) k_asm_fluid(AsmArgs A) {
   // sums over the points: of rV2, pa and, for the first three nodes, of the
   // gradient part of lR (gR) and of up.Nx_a (sU); lN: rd rV2 at node g
   double vS[3] = {0, 0, 0}, paS = 0.0, gR[3][3], sU[3] = {0, 0, 0}, lN[4][3];
-  // tangent factors (first three nodes): Q = sum tauM uaNx, QU = sum tauM uNx,
-  // UA = sum uaNx, H = the two quadratic sums of S_ab; q2[a][g] = (tauM uaNx_a)
-  // and u2[g][b] = uaNx_b at point g, tMg = tauM at point g
+  // tangent factors (of the first NA nodes): Q = sum tauM uaNx, QU = sum tauM
+  // uNx, UA = sum uaNx, H = the two quadratic sums of S_ab; q2[a][g] = (tauM
+  // uaNx_a) and u2[g][b] = uaNx_b at point g, tMg = tauM at point g
+  constexpr int NA = sizeof(TT) == 4 ? 4 : 3;
   const TT rh = TT(rho), rh2 = rh * rh, md = TT(A.fl_amd);
-  TT SC = TT(0), ST = TT(0), Q[3], QU[3], UA[3], H[3][3], q2[3][4], u2[4][3], tMg[4];
+  TT SC = TT(0), ST = TT(0), Q[NA], QU[NA], UA[NA], H[NA][NA], q2[NA][4], u2[4][NA], tMg[4];
 #pragma unroll
-  for (int a = 0; a < 3; a++) {
+  for (int a = 0; a < NA; a++) {
     Q[a] = QU[a] = UA[a] = TT(0);
 #pragma unroll
-    for (int b = 0; b < 3; b++) {
-      H[a][b] = TT(0);
-      gR[a][b] = 0.0;
-    }
+    for (int b = 0; b < NA; b++) H[a][b] = TT(0);
   }
+#pragma unroll
+  for (int a = 0; a < 3; a++)
+#pragma unroll
+    for (int b = 0; b < 3; b++) gR[a][b] = 0.0;
 #pragma unroll
   for (int g = 0; g < 4; g++) {
     double u[3], uN[3], rV[3], up[3], upN[3];
@@ -193,15 +199,19 @@ __global__ void __launch_bounds__(kAsmThreads) k_asm_fluid(AsmArgs A) {
     SC += TT(tauC);
     ST += tM;
     tMg[g] = tM;
-    TT un[3], pn[3];
+    TT un[NA], pn[NA];
 #pragma unroll
     for (int a = 0; a < 3; a++) {
       sU[a] += upN[a];
       un[a] = TT(uN[a]);
       pn[a] = TT(upN[a]);
     }
+    if constexpr (NA == 4) {
+      un[3] = TT(u[0] * Nx[0][3] + u[1] * Nx[1][3] + u[2] * Nx[2][3]);
+      pn[3] = TT(up[0] * Nx[0][3] + up[1] * Nx[1][3] + up[2] * Nx[2][3]);
+    }
 #pragma unroll
-    for (int a = 0; a < 3; a++) {
+    for (int a = 0; a < NA; a++) {
       const TT ua = un[a] + pn[a], ta = tM * ua;
       Q[a] += ta;
       QU[a] += tM * un[a];
@@ -210,7 +220,7 @@ __global__ void __launch_bounds__(kAsmThreads) k_asm_fluid(AsmArgs A) {
       u2[g][a] = ua;
       const TT c1 = rh2 * ta, c3 = tB * pn[a];
 #pragma unroll
-      for (int b = 0; b < 3; b++) H[a][b] += c1 * un[b] + c3 * pn[b];
+      for (int b = 0; b < NA; b++) H[a][b] += c1 * un[b] + c3 * pn[b];
     }
   }
   // lR(a,j) = wr (rt sum_g rV2_j + rd rV2_j(a)) + w [4 mu es.Nx_a + gR - paS Nx_a]_j,
@@ -252,23 +262,30 @@ __global__ void __launch_bounds__(kAsmThreads) k_asm_fluid(AsmArgs A) {
   const TT w2 = wlt * rh2 * md;
   TT S[4][4];
 #pragma unroll
-  for (int a = 0; a < 3; a++)
+  for (int a = 0; a < NA; a++)
 #pragma unroll
     for (int b = 0; b < 4; b++) S[a][b] = w2 * (trt * Q[a] + trd * q2[a][b]);
+  if constexpr (NA == 3) {
 #pragma unroll
-  for (int b = 0; b < 4; b++) S[3][b] = -(S[0][b] + S[1][b] + S[2][b]);
+    for (int b = 0; b < 4; b++) S[3][b] = -(S[0][b] + S[1][b] + S[2][b]);
+  }
 #pragma unroll
   for (int a = 0; a < 4; a++) {
     TT s4 = TT(0);
 #pragma unroll
-    for (int b = 0; b < 3; b++) {
+    for (int b = 0; b < NA; b++) {
       const TT v = wrh * (trt * UA[b] + trd * u2[a][b]);
       S[a][b] += v;
       s4 -= v;
     }
-    S[a][3] += s4;
+    if constexpr (NA == 3) S[a][3] += s4;
   }
-  {
+  if constexpr (NA == 4) {
+#pragma unroll
+    for (int a = 0; a < 4; a++)
+#pragma unroll
+      for (int b = 0; b < 4; b++) S[a][b] += wlt * H[a][b];
+  } else {
     TT h3[4] = {TT(0), TT(0), TT(0), TT(0)};
 #pragma unroll
     for (int a = 0; a < 3; a++) {
@@ -290,8 +307,8 @@ __global__ void __launch_bounds__(kAsmThreads) k_asm_fluid(AsmArgs A) {
   TT Qw[4], Vw[4];
 #pragma unroll
   for (int a = 0; a < 4; a++) {
-    const TT qa = a < 3 ? Q[a < 3 ? a : 0] : -(Q[0] + Q[1] + Q[2]);
-    const TT qu = a < 3 ? QU[a < 3 ? a : 0] : -(QU[0] + QU[1] + QU[2]);
+    const TT qa = a < NA ? Q[a < NA ? a : 0] : -(Q[0] + Q[1] + Q[2]);
+    const TT qu = a < NA ? QU[a < NA ? a : 0] : -(QU[0] + QU[1] + QU[2]);
     Qw[a] = wrh * qa;
     Vw[a] = wrh * (qu + md * (trt * ST + trd * tMg[a]));
   }

@@ -67,7 +67,7 @@ def parts(phys, V):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("apex", [0, 1, 2, 3])
-@pytest.mark.parametrize("phys", ["struct", "lelas", "heatf"])
+@pytest.mark.parametrize("phys", ["struct", "lelas", "fluid", "heatf"])
 def test_smallest_gradient_keeps_its_digits(gsls, phys, apex):
     torch = pytest.importorskip("torch")
     p = needle(phys, apex)
