@@ -39,21 +39,23 @@ __host__ __device__ __forceinline__ void fix_limbs(unsigned long long bits, int 
   S[2] = (s2 ^ sg) - sg;
 }
 
+// hi 2^23 + lo, 0 <= lo < 2^23, shifted down by sh >= 0 bits with floor
+__host__ __device__ __forceinline__ void fix_down(long long &hi, int &lo, int sh) {
+  if (sh < 23) {
+    lo = (int)((((unsigned long long)hi << (23 - sh)) & kFixMask) | (unsigned)(lo >> sh));
+  } else {
+    lo = (int)((hi >> (sh - 23 < 63 ? sh - 23 : 63)) & kFixMask);
+  }
+  hi >>= sh < 63 ? sh : 63;
+}
+
 // a block sum (e; S2, S1, S0) relative to E >= e: hi 2^23 + lo, 0 <= lo < 2^23,
 // |hi| < 2^55 (shifted down with floor)
 __host__ __device__ __forceinline__ void fix_align(int e, const int S[3], int E, long long &hi,
                                                    int &lo) {
   hi = (long long)S[2] * (1 << 23) + S[1] + (S[0] >> 23);
   lo = S[0] & kFixMask;
-  const int sh = E - e;
-  if (sh > 0) {
-    if (sh < 23) {
-      lo = (int)(((hi << (23 - sh)) & kFixMask) | (lo >> sh));
-    } else {
-      lo = (int)((hi >> (sh - 23 < 63 ? sh - 23 : 63)) & kFixMask);
-    }
-    hi >>= sh < 63 ? sh : 63;
-  }
+  fix_down(hi, lo, E - e);
 }
 
 // (hi 2^23 + lo) 2^(E - 1091) rounded to nearest; |hi| < 2^62, 0 <= lo < 2^31

@@ -162,9 +162,9 @@ static __device__ __noinline__ double grid_red_total(GridRed g, unsigned epoch, 
     e = __reduce_max_sync(0xffffffffu, e);
     if (k0 > 0 && e > E) {
       // the sum of the earlier turns, relative to the larger exponent
-      const int sh = min(e - E, 63);
-      Lo = sh < 23 ? (unsigned)(((H << (23 - sh)) & kFixMask) | (Lo >> sh)) : 0u;
-      H >>= sh;
+      int lo = (int)Lo;
+      fix_down(H, lo, e - E);
+      Lo = (unsigned)lo;
     }
     E = e;
 #pragma unroll 1
