@@ -48,6 +48,27 @@ struct PartArgs {
 int part_setup(gsls_lhs *lhs);
 PartArgs part_args(const RowPart &p);
 
+// Most dynamic shared memory of a block of the kernel on this device
+inline size_t smem_cap(const void *kernel) {
+  int dev = 0, opt = 0;
+  cudaFuncAttributes fa{};
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&opt, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+  if (cudaFuncGetAttributes(&fa, kernel) != cudaSuccess) return 0;
+  return (size_t)opt - fa.sharedSizeBytes;
+}
+
+// Cooperative launch with smem bytes of dynamic shared memory.  The attribute
+// that allows them belongs to the kernel, not to the launch: it is always set
+// to the same value, the most there is (cap), so that of two host threads with
+// systems of different size neither lowers it between the other's two calls.
+inline int coop_launch(const void *kernel, size_t cap, int nblk, void **args, size_t smem,
+                       cudaStream_t st) {
+  GSLS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cap));
+  GSLS_CUDA(cudaLaunchCooperativeKernel(kernel, dim3(nblk), dim3(kPartThreads), args, smem, st));
+  return GSLS_OK;
+}
+
 // A node's D values in global memory, read and written through L2; stride VD
 // (3-vectors are padded to 4 values: whole 16-byte accesses)
 template <int D, class XT>

@@ -440,18 +440,18 @@ __global__ void __launch_bounds__(kPartThreads, 1) k_wcg(WcgArgs<XT> A) {
   if (threadIdx.x == 0 && !ok) atomicExch(&A.red.buf->bar.err, 1);
 }
 
+// Most dynamic shared memory of a block of the kernel
+template <int D, class VT, class XT>
+static size_t wcg_cap() {
+  static const size_t cap = [] { return smem_cap((const void *)k_wcg<D, VT, XT>); }();
+  return cap;
+}
+
 // Shared memory of the kernel: the window and KP; R of the own rows, then X,
 // where they fit too.  0: the window does not fit.
 template <int D, class VT, class XT>
 static size_t wcg_geometry(const PartArgs &P, WcgArgs<XT> &A) {
-  static const size_t cap = [] {
-    int dev = 0, opt = 0;
-    cudaFuncAttributes fa{};
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&opt, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    if (cudaFuncGetAttributes(&fa, k_wcg<D, VT, XT>) != cudaSuccess) return (size_t)0;
-    return (size_t)opt - fa.sharedSizeBytes;
-  }();
+  const size_t cap = wcg_cap<D, VT, XT>();
   const auto up16 = [](size_t n) { return (n + 15) & ~(size_t)15; };
   A.ownMax = P.nslMax * (32 / P.L);
   const size_t own1 = (size_t)A.ownMax * D * sizeof(XT);
@@ -477,8 +477,6 @@ static int wcg_t(gsls_lhs *lhs, gsls_sub_ls *ls, const VT *Val, double *R, const
   WcgArgs<XT> A{};
   const size_t smem = wcg_geometry<D, VT, XT>(P, A);
   if (!smem) return GSLS_OK;
-  GSLS_CUDA(cudaFuncSetAttribute(k_wcg<D, VT, XT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem));
   *ran = true;
   const size_t vb = ((size_t)P.nslots * NodeL2<D, XT>::VD * sizeof(XT) + 127) & ~(size_t)127;
   GSLS_TRY(ws.wcg_stream.alloc(Rec<D, VT>::at(P.nsteps, P.nblk * kPartWarps)));
@@ -515,8 +513,8 @@ static int wcg_t(gsls_lhs *lhs, gsls_sub_ls *ls, const VT *Val, double *R, const
   void *args[] = {&A};
   const bool prof = prof_on();
   if (prof) cudaEventRecord(prof_event(0), st);
-  GSLS_CUDA(cudaLaunchCooperativeKernel((const void *)k_wcg<D, VT, XT>, dim3(P.nblk),
-                                        dim3(kPartThreads), args, smem, st));
+  GSLS_TRY(coop_launch((const void *)k_wcg<D, VT, XT>, wcg_cap<D, VT, XT>(), P.nblk, args, smem,
+                       st));
   GSLS_CHECK_LAUNCH();
   if (prof) cudaEventRecord(prof_event(1), st);
   // the error word travels behind the scalars

@@ -352,21 +352,19 @@ static size_t wschur_smem(const RowPart &p) {
          sizeof(int) * (size_t)kPartWarps * grp_cap(p.nslMax, p.grpMax, SRec<3, XT>::G);
 }
 
+template <class VT, class XT>
+static size_t wschur_cap() {
+  static const size_t cap = [] { return smem_cap((const void *)k_wschur<VT, XT>); }();
+  return cap;
+}
+
 template <class VT>
 int wschur_pack(gsls_lhs *lhs, const VT *mG, const VT *Gt, const VT *mL, bool *fits) {
   *fits = false;
   Workspace &ws = lhs->ws;
   GSLS_TRY(part_setup(lhs));
   if (!ws.part.ok) return GSLS_OK;
-  static const size_t cap = [] {
-    int dev = 0, opt = 0;
-    cudaFuncAttributes fa{};
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&opt, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    if (cudaFuncGetAttributes(&fa, k_wschur<VT, VT>) != cudaSuccess) return (size_t)0;
-    return (size_t)opt - fa.sharedSizeBytes;
-  }();
-  if (wschur_smem<VT>(ws.part) > cap) return GSLS_OK;
+  if (wschur_smem<VT>(ws.part) > wschur_cap<VT, VT>()) return GSLS_OK;
   const PartArgs P = part_args(ws.part);
   const size_t n1 = (size_t)P.nsteps8 * SRec<3, VT>::SB, n2 = (size_t)P.nsteps8 * SRec<4, VT>::SB;
   const size_t vb = ((size_t)P.nslots * sizeof(VT) + 127) & ~(size_t)127;
@@ -391,8 +389,6 @@ int wschur_run(gsls_lhs *lhs, const gsls_sub_ls *ls, XT *x, SchurScal *out) {
   unsigned char *s1 = ws.ns_stream.as<unsigned char>();
   unsigned char *sc = ws.scal.as<unsigned char>();
   const size_t smem = wschur_smem<XT>(ws.part);
-  GSLS_CUDA(cudaFuncSetAttribute(k_wschur<VT, XT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem));
   GSLS_CUDA(cudaMemsetAsync(sc + kScalRed, 0, sizeof(GridBar), st));
   WschurArgs<XT> A{};
   A.P = P;
@@ -411,8 +407,8 @@ int wschur_run(gsls_lhs *lhs, const gsls_sub_ls *ls, XT *x, SchurScal *out) {
   void *args[] = {&A};
   const bool prof = prof_on();
   if (prof) cudaEventRecord(prof_event(0), st);
-  GSLS_CUDA(cudaLaunchCooperativeKernel((const void *)k_wschur<VT, XT>, dim3(P.nblk),
-                                        dim3(kPartThreads), args, smem, st));
+  GSLS_TRY(coop_launch((const void *)k_wschur<VT, XT>, wschur_cap<VT, XT>(), P.nblk, args, smem,
+                       st));
   GSLS_CHECK_LAUNCH();
   if (prof) cudaEventRecord(prof_event(1), st);
   // the error word travels behind the scalars
