@@ -94,6 +94,15 @@ int gsls_init(int device);
    returns GSLS_ERR_CUDA with the CUDA context intact.  A test hook for the
    timeout path; a small limit makes waits expire on healthy launches. */
 int gsls_set_wait_limit(unsigned polls);
+/* No counterpart in the reference.  Device memory that the library may still
+   take for the calling thread: a request above it fails as on a device that
+   is out of memory, what the thread frees counts as free again; a negative
+   value (the default) sets no budget.  A test hook for the paths that a
+   device short of memory takes. */
+int gsls_set_alloc_budget(long long bytes);
+/* Device memory requests of the library so far, and the bytes it holds. */
+long long gsls_alloc_count(void);
+long long gsls_alloc_bytes(void);
 /* Library version (GSLS_VERSION). */
 int gsls_version(void);
 /* Human-readable text for the last error of this thread. */

@@ -39,7 +39,8 @@ struct gsls_mesh {
     gsls::DevBuf ptr, ent;
   };
   std::vector<std::unique_ptr<Inverse>> inv;
-  gsls::DevBuf d_elK, d_elR;
+  gsls::DevBuf d_el;
+  size_t el_most = 0;             // most bytes of d_el (0: not asked for yet)
   bool inv_ready = false;
   std::mutex el_mu;               // held while an assembly through the buffer is enqueued
   gsls::DevBuf d_geo;             // per-element Nx (12) and Jacobian, SoA: geo[k * nEl + e]
@@ -540,17 +541,26 @@ static int assemble_gather(gsls_mesh *m, K kern, size_t smem, AsmArgs A, double 
   constexpr int DD = DOF * DOF;
   gsls_lhs *lhs = m->lhs;
   cudaStream_t st = lhs->stream;
-  const size_t per = 16 * DD * sizeof(VT) + 4 * DOF * sizeof(double);
-  int part = (int)std::min<size_t>((size_t)m->nEl, kElemBuf / per);
-  // a device short of memory takes smaller parts
-  while (m->d_elK.alloc(16 * DD * sizeof(VT) * (size_t)part) != GSLS_OK ||
-         m->d_elR.alloc(4 * DOF * sizeof(double) * (size_t)part) != GSLS_OK) {
-    cudaGetLastError();
-    if (part <= 4096) return GSLS_ERR_CUDA;
-    part /= 2;
+  // matrices, then residuals (4 * DOF doubles: whole 16-byte vectors).  At most
+  // a quarter of the free memory, since a solver's workspaces are taken later;
+  // smaller parts still where that cannot be had.  The size that was had is
+  // kept: asking for more again would free the buffer each time.
+  constexpr size_t kEl = 16 * DD * sizeof(VT), kRes = 4 * DOF * sizeof(double);
+  constexpr size_t per = kEl + kRes;
+  static_assert(kEl % 16 == 0 && kRes % 16 == 0, "whole vectors");
+  if (m->el_most == 0)
+    m->el_most = std::max(std::min(kElemBuf, mem_free() / 4), (size_t)4096 * per);
+  for (size_t n = per * std::min((size_t)m->nEl, m->el_most / per); !m->d_el.try_alloc(n);) {
+    if (n <= 4096 * per) {
+      m->el_most = 0;
+      return GSLS_ERR_CUDA;
+    }
+    n = std::max(n / 2, (size_t)4096 * per);
+    m->el_most = n;
   }
-  A.lK = m->d_elK.p;
-  A.lR = m->d_elR.as<double>();
+  const int part = (int)std::min<size_t>((size_t)m->nEl, m->d_el.bytes / per);
+  A.lK = m->d_el.p;
+  A.lR = reinterpret_cast<double *>(m->d_el.as<unsigned char>() + kEl * (size_t)part);
   const size_t sm = smem * (kAsmThreads / 32);
   if (sm > 48 * 1024)
     GSLS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
@@ -566,10 +576,10 @@ static int assemble_gather(gsls_mesh *m, K kern, size_t smem, AsmArgs A, double 
     const size_t n = (size_t)lhs->nnz * (DD / gather_width<DD, VT>());
     const unsigned gv = (unsigned)std::min<size_t>((n + 255) / 256, 1u << 20);
     if (ne == m->nEl)
-      k_gather_val<DD, VT, false><<<gv, 256, 0, st>>>(n, ptr, ent, m->d_elK.as<VT>(), f, f + ne,
+      k_gather_val<DD, VT, false><<<gv, 256, 0, st>>>(n, ptr, ent, m->d_el.as<VT>(), f, f + ne,
                                                       1, Val);
     else
-      k_gather_val<DD, VT, true><<<gv, 256, 0, st>>>(n, ptr, ent, m->d_elK.as<VT>(), f, f + ne,
+      k_gather_val<DD, VT, true><<<gv, 256, 0, st>>>(n, ptr, ent, m->d_el.as<VT>(), f, f + ne,
                                                      e0 == 0, Val);
     GSLS_CHECK_LAUNCH();
     k_gather_res<DOF><<<(lhs->nNo * DOF + 255) / 256, 256, 0, st>>>(

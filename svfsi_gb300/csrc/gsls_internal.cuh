@@ -59,7 +59,8 @@ void prof_add(const char *name, long long count, double ms);
 cudaEvent_t prof_event(int i);
 
 // ---------------------------------------------------------------------------
-// device buffer (RAII, stream-ordered free)
+// device buffer (RAII, stream-ordered free); a failed alloc leaves it empty
+size_t mem_free();  // device memory that a DevBuf could take now
 struct DevBuf {
   void *p = nullptr;
   size_t bytes = 0;
@@ -68,6 +69,7 @@ struct DevBuf {
   DevBuf &operator=(const DevBuf &) = delete;
   ~DevBuf() { release(); }
   int alloc(size_t n);              // no-op if already >= n bytes
+  bool try_alloc(size_t n);         // the same; false when the memory could not be had
   void release();
   template <class T> T *as() const { return reinterpret_cast<T *>(p); }
 };
@@ -165,6 +167,7 @@ struct Workspace {
   unsigned long long wcg_serial = 0;  // preconditioning whose matrix the stream holds
   const void *wcg_val = nullptr;      // (and the array it was packed from)
   int wcg_key = 0;                    // block size and value type of the stream
+  size_t wcg_short = SIZE_MAX;        // stream size that could not be had
   DevBuf x32;         // FP32 copy of the vector of gsls_spmv_dev
   std::mutex x32_mu;  // held while the copy and the product that reads it are enqueued
   DevBuf partials;    // double[grid * 64]
@@ -180,6 +183,7 @@ struct Workspace {
   DevBuf io2;
   DevBuf ns_vec;      // NS solver vectors (Rm, Rc, U, P, MU, MP, Schur CG)
   DevBuf ns_stream;   // streams and published vectors of the Schur CG (gsls_wschur.cu)
+  size_t ns_short = SIZE_MAX;  // size of ns_stream that could not be had
   DevBuf ns_mat;      // NS solver blocks (mK, mG, mD, mL, Gt)
   DevBuf rcs;         // RCS scaling state (W1, Wr, Wc, control words)
   DevBuf cpl_glob, cpl_valM;  // coupled faces of the current solve
@@ -390,7 +394,8 @@ template <class XT>
 void launch_addbcmul(gsls_lhs *lhs, int op, int vdof, const XT *X, XT *Y, const int *done);
 // CG on the preconditioned system as one cooperative launch (gsls_wcg.cu);
 // R in: rhs, out: W X.  keep: Val is what the last preconditioning on this
-// lhs left.  *ran false: the partition's windows do not fit, nothing done.
+// lhs left.  *ran false: the partition's windows do not fit in shared memory
+// or its tables and stream in device memory; nothing done.
 int wcg_run(gsls_lhs *lhs, gsls_sub_ls *ls, int D, bool mixed, const void *Val, double *R,
             const double *W, bool keep, bool *ran);
 // BiCGStab on the preconditioned system (gsls_bicgs.cu)

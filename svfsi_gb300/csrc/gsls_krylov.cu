@@ -957,12 +957,13 @@ static int cg_t(gsls_lhs *lhs, gsls_sub_ls *ls, const VT *Val, double *R, const 
   // Sliced SpMV: a solve that is still running after its first batch packs
   // the matrix into the sliced layout (one pass over Val) and continues on
   // it; short solves (a few iterations) never pay for the copy.
-  // GSLS_SPMV=csr keeps the CSR kernel throughout.
+  // GSLS_SPMV=csr keeps the CSR kernel throughout, as does a device that had no
+  // memory for the partition's stream, the other copy of the matrix.
   static const bool want_sell = [] {
     const char *e = getenv("GSLS_SPMV");
     return !(e && (strcmp(e, "csr") == 0 || strcmp(e, "tma") == 0));
   }();
-  const bool sell_ok = want_sell && !FUSED && !use_tma;
+  const bool sell_ok = want_sell && !FUSED && !use_tma && ws.wcg_short == SIZE_MAX;
   SellArgs sa{};
   bool sell_on = false;
   // First batch: the smallest power of two that holds the previous solve's

@@ -13,6 +13,8 @@ namespace gsls {
 
 static thread_local std::string g_err;
 static std::atomic<long long> g_launches{0};
+static std::atomic<long long> g_allocs{0}, g_bytes{0};
+static thread_local long long t_budget = -1;  // gsls_set_alloc_budget
 
 void set_error(const std::string &msg) { g_err = msg; }
 
@@ -85,18 +87,37 @@ int DevBuf::alloc(size_t n) {
   if (n <= bytes && p) return GSLS_OK;
   release();
   if (n == 0) n = 16;
-  cudaError_t e = cudaMalloc(&p, n);
+  const bool over = t_budget >= 0 && n > (size_t)t_budget;
+  cudaError_t e = over ? cudaErrorMemoryAllocation : cudaMalloc(&p, n);
+  g_allocs.fetch_add(1, std::memory_order_relaxed);
   if (e != cudaSuccess) {
     p = nullptr;
-    bytes = 0;
     return cuda_fail(e, "cudaMalloc", __FILE__, __LINE__);
   }
   bytes = n;
+  g_bytes.fetch_add((long long)n, std::memory_order_relaxed);
+  if (t_budget >= 0) t_budget -= (long long)n;
   return GSLS_OK;
 }
 
+bool DevBuf::try_alloc(size_t n) {
+  if (alloc(n) == GSLS_OK) return true;
+  cudaGetLastError();  // the caller has another way
+  return false;
+}
+
+size_t mem_free() {
+  size_t f = 0, t = 0;
+  if (cudaMemGetInfo(&f, &t) != cudaSuccess) f = 0;
+  return t_budget >= 0 && (size_t)t_budget < f ? (size_t)t_budget : f;
+}
+
 void DevBuf::release() {
-  if (p) cudaFree(p);
+  if (p) {
+    cudaFree(p);
+    g_bytes.fetch_sub((long long)bytes, std::memory_order_relaxed);
+    if (t_budget >= 0) t_budget += (long long)bytes;
+  }
   p = nullptr;
   bytes = 0;
 }
@@ -447,6 +468,15 @@ int gsls_profile_read(const char *name, long long *count, double *total_ms) {
   if (total_ms) *total_ms = 0.0;
   return GSLS_OK;
 }
+
+int gsls_set_alloc_budget(long long bytes) {
+  t_budget = bytes;
+  return GSLS_OK;
+}
+
+long long gsls_alloc_count(void) { return g_allocs.load(); }
+
+long long gsls_alloc_bytes(void) { return g_bytes.load(); }
 
 int gsls_set_wait_limit(unsigned polls) {
   g_wait_limit.store(polls ? polls : kBarSpinDefault, std::memory_order_relaxed);

@@ -294,7 +294,11 @@ static int part_build(gsls_lhs *lhs, RowPart &p) {
     p.off[7] = append(img, H.lcol);
     p.off[8] = append(img, H.sst);
     p.off[9] = append(img, H.soff);
-    GSLS_TRY(p.buf.alloc(img.size() + 16));
+    if (!p.buf.try_alloc(img.size() + 16)) {
+      p.ok = false;
+      p.built = true;
+      return GSLS_OK;
+    }
     GSLS_CUDA(cudaMemcpyAsync(p.buf.p, img.data(), img.size(), cudaMemcpyHostToDevice,
                               lhs->stream));
     GSLS_CUDA(cudaStreamSynchronize(lhs->stream));  // img goes out of scope
@@ -319,8 +323,9 @@ int part_setup(gsls_lhs *lhs) {
   try {
     return part_build(lhs, p);
   } catch (const std::bad_alloc &) {
-    set_error("row partition: out of host memory");
-    return GSLS_ERR_NOMEM;
+    p.ok = false;
+    p.built = true;
+    return GSLS_OK;
   }
 }
 

@@ -44,7 +44,8 @@ struct PartArgs {
 };
 
 // Partition of the lhs over at most num_sms() blocks; built on the host once
-// per lhs.  ok is false when a window has more than 65,535 entries.
+// per lhs.  ok is false when a window has more than 65,535 entries or there is
+// no memory for the tables: the callers then have kernels without them.
 int part_setup(gsls_lhs *lhs);
 PartArgs part_args(const RowPart &p);
 

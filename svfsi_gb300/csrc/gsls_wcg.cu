@@ -477,10 +477,19 @@ static int wcg_t(gsls_lhs *lhs, gsls_sub_ls *ls, const VT *Val, double *R, const
   WcgArgs<XT> A{};
   const size_t smem = wcg_geometry<D, VT, XT>(P, A);
   if (!smem) return GSLS_OK;
-  *ran = true;
   const size_t vb = ((size_t)P.nslots * NodeL2<D, XT>::VD * sizeof(XT) + 127) & ~(size_t)127;
-  GSLS_TRY(ws.wcg_stream.alloc(Rec<D, VT>::at(P.nsteps, P.nblk * kPartWarps)));
-  GSLS_TRY(ws.wcg_vec.alloc(2 * vb));
+  const size_t sb = Rec<D, VT>::at(P.nsteps, P.nblk * kPartWarps);
+  // no memory for a second copy of the matrix: the batched kernels take the
+  // solve, and later ones of that size without another try
+  if (sb >= ws.wcg_short) return GSLS_OK;
+  if (!ws.wcg_stream.try_alloc(sb) || !ws.wcg_vec.try_alloc(2 * vb)) {
+    ws.wcg_stream.release();
+    ws.wcg_vec.release();
+    ws.wcg_key = 0;
+    ws.wcg_short = sb;
+    return GSLS_OK;
+  }
+  *ran = true;
   const int key = D * 16 + (int)sizeof(VT);
   // keep: Val is the matrix that the last preconditioning on this lhs left
   // (no other call can have changed it), so its stream is packed already

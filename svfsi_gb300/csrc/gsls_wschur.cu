@@ -368,7 +368,13 @@ int wschur_pack(gsls_lhs *lhs, const VT *mG, const VT *Gt, const VT *mL, bool *f
   const PartArgs P = part_args(ws.part);
   const size_t n1 = (size_t)P.nsteps8 * SRec<3, VT>::SB, n2 = (size_t)P.nsteps8 * SRec<4, VT>::SB;
   const size_t vb = ((size_t)P.nslots * sizeof(VT) + 127) & ~(size_t)127;
-  GSLS_TRY(ws.ns_stream.alloc(n1 + n2 + 5 * vb + 512));
+  // no memory for the streams: the per-kernel Schur CG, without another try
+  const size_t sb = n1 + n2 + 5 * vb + 512;
+  if (sb >= ws.ns_short) return GSLS_OK;
+  if (!ws.ns_stream.try_alloc(sb)) {
+    ws.ns_short = sb;
+    return GSLS_OK;
+  }
   unsigned char *s1 = ws.ns_stream.as<unsigned char>(), *s2 = s1 + ((n1 + 127) & ~(size_t)127);
   k_wschur_pack<3, VT><<<8 * num_sms(), 256, 0, lhs->stream>>>(P, mG, nullptr, s1);
   GSLS_CHECK_LAUNCH();
