@@ -144,6 +144,9 @@ struct GraphKey {
   }
 };
 
+// matrix values from which gsls_spmv_dev rounds its vector to FP32 once
+constexpr long long kX32Values = 2 << 20;
+
 // Scratch for reductions and Krylov work vectors.
 struct Workspace {
   DevBuf Wf;          // float copy of W (FP32 scaling pass)
@@ -168,8 +171,6 @@ struct Workspace {
   const void *wcg_val = nullptr;      // (and the array it was packed from)
   int wcg_key = 0;                    // block size and value type of the stream
   size_t wcg_short = SIZE_MAX;        // stream size that could not be had
-  DevBuf x32;         // FP32 copy of the vector of gsls_spmv_dev
-  std::mutex x32_mu;  // held while the copy and the product that reads it are enqueued
   DevBuf partials;    // double[grid * 64]
   DevBuf ticket;      // unsigned[8]
   DevBuf scal;        // KrylovScalars; then GridRedBuf
@@ -204,6 +205,11 @@ struct gsls_lhs {
   gsls::DevBuf d_rowPtr, d_colPtr, d_diagPtr, d_rowOf;
   gsls::DevBuf d_tpos;   // CSR position of the transposed block (built on first use)
   bool tpos_ok = false;
+  // FP32 copy of the vector of gsls_spmv_dev (up to 4 values per node, behind
+  // d_diagPtr), and the mutex held while the copy and the product that reads it
+  // are enqueued
+  float *x32 = nullptr;
+  std::mutex x32_mu;
   std::vector<gsls::Face> faces;
   cudaStream_t stream = nullptr;
   bool own_stream = false;

@@ -1188,12 +1188,11 @@ static int spmv_t(gsls_lhs *lhs, const void *dVal, bool mixed, const double *x, 
   // conversion per matrix value, ~0.55 T/s: 2.5 us at 2^21 / 1.5 values; the
   // 3x3 beam of 47 M values 119 -> 68 us, of which 32 us are its bytes at the
   // HBM copy rate)
-  if ((long long)lhs->nnz * D * D < (2 << 20))
+  if ((long long)lhs->nnz * D * D < kX32Values)
     return spmv_ln<D, D>(lhs, (const float *)dVal, x, y, false);
   constexpr int VD = VStride<D, float>::v;
-  std::lock_guard<std::mutex> lk(lhs->ws.x32_mu);
-  GSLS_TRY(lhs->ws.x32.alloc(sizeof(float) * (size_t)lhs->nNo * VD));
-  float *xf = lhs->ws.x32.as<float>();
+  std::lock_guard<std::mutex> lk(lhs->x32_mu);
+  float *xf = lhs->x32;
   k_x32<D, VD><<<blocks_for(lhs->nNo, num_sms() * 8), 256, 0, lhs->stream>>>(lhs->nNo, x, xf);
   GSLS_CHECK_LAUNCH();
   return spmv_ln<D, VD>(lhs, (const float *)dVal, (const float *)xf, y, true);

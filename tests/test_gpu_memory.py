@@ -5,7 +5,7 @@ do not ask for the same memory again on every call.
 The library is given a budget (gsls_set_alloc_budget) in place of a full
 device.  Tolerances: the solves stop at 1e-10 |r0| on systems with a condition
 number below 5 (as in test_gpu_wcg.py); an assembly in parts has the bits of
-the whole one, since a block's sum keeps its order; steps of the NS solver
+the whole one, since a block's sum keeps its order; sums of ones are exact; steps of the NS solver
 on either Schur CG stop at 1e-10 of the first residual.
 """
 import ctypes as C
@@ -121,6 +121,26 @@ def test_schur_cg_without_memory_for_the_streams(gsls, budget):
     # both stop at 1e-10 of the first residual
     for y in Y[1:]:
         assert np.linalg.norm(y - Y[0]) <= 1e-7 * np.linalg.norm(Y[0])
+
+
+@pytest.mark.parametrize("d", [1, 3, 4])
+def test_spmv_asks_for_no_memory(gsls, d):
+    """The room for an FP32 copy of the vector comes with the lhs."""
+    torch = pytest.importorskip("torch")
+    rp, cp = _graph(("box", 100, 25, 25) if d < 4 else ("box", 60, 15, 15))
+    n = rp.size - 1
+    lhs = fsils.FSILS_LHS_CREATE(n, n, cp.size, np.arange(1, n + 1, dtype=np.int32),
+                                 rp.astype(np.int32) + 1, cp.astype(np.int32) + 1, 1)
+    dV = torch.ones(cp.size * d * d + 8, dtype=torch.float32, device="cuda")
+    dx = torch.ones(n * d, dtype=torch.float64, device="cuda")
+    dy = torch.empty_like(dx)
+    torch.cuda.synchronize()
+    a0 = gsls.gsls_alloc_count()
+    _lib.check(gsls.gsls_spmv_dev(lhs.h, d, C.c_void_p(dV.data_ptr()), fsils.PREC_MIXED,
+                                  C.c_void_p(dx.data_ptr()), C.c_void_p(dy.data_ptr())))
+    assert gsls.gsls_alloc_count() == a0
+    assert np.array_equal(dy.cpu().numpy().reshape(n, d)[:, 0], np.diff(rp) * d)
+    lhs.free()
 
 
 @pytest.mark.parametrize("phys", ["struct", "fluid"])
