@@ -89,25 +89,6 @@ __global__ void k_inv_count(size_t n, const int *__restrict__ map, int *__restri
 // exclusive scan in three launches: sums of chunks of kScan, of the chunk
 // sums (one block), and within the chunks
 constexpr int kScan = 2048;
-__device__ __forceinline__ int block_scan_excl(int v, int *sh, int &total) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  int x = v;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int y = __shfl_up_sync(0xffffffffu, x, o);
-    if (lane >= o) x += y;
-  }
-  __syncthreads();
-  if (lane == 31) sh[wid] = x;
-  __syncthreads();
-  int base = 0;
-  total = 0;
-  for (int k = 0; k < nw; k++) {
-    if (k < wid) base += sh[k];
-    total += sh[k];
-  }
-  return base + x - v;
-}
 __global__ void __launch_bounds__(256) k_scan_sums(int n, const int *__restrict__ cnt,
                                                    int *__restrict__ sums) {
   __shared__ int sh[32];

@@ -101,8 +101,11 @@ struct RowPart {
   bool built = false, ok = false;
   int nblk = 0, L = 1, winMax = 0, nslMax = 0, stMax = 0, grpMax = 0, nS = 0;
   long long slots = 0, steps = 0, steps8 = 0;
-  DevBuf buf;           // the tables of PartArgs at their offsets
-  size_t off[10] = {};
+  DevBuf buf;             // the tables per slot, slice and block, at their offsets
+  size_t off[7] = {};
+  std::vector<int> hoff;  // halo offsets
+  DevBuf tab;             // halos, sources and columns of the steps (part_fill)
+  DevBuf tmp;             // the halos as bits, until tab is filled
 };
 
 // Face (BC) description, FSILS_faceType.
@@ -257,6 +260,27 @@ __device__ __forceinline__ double block_sum(double v, double *sh /*[32]*/) {
   v = (threadIdx.x < nw) ? sh[threadIdx.x] : 0.0;
   if (wid == 0) v = warp_sum(v);
   return v;
+}
+
+// exclusive prefix sum over the block and its total; sh[32]
+__device__ __forceinline__ int block_scan_excl(int v, int *sh, int &total) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  int x = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
+  }
+  __syncthreads();
+  if (lane == 31) sh[wid] = x;
+  __syncthreads();
+  int base = 0;
+  total = 0;
+  for (int k = 0; k < nw; k++) {
+    if (k < wid) base += sh[k];
+    total += sh[k];
+  }
+  return base + x - v;
 }
 
 // Ticket increment with acquire-release semantics at GPU scope: the

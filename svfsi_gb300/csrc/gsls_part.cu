@@ -1,4 +1,9 @@
-// Host construction of the row partition (gsls_part.cuh).
+// Construction of the row partition (gsls_part.cuh): the rows of each block on
+// the host, the halos and columns on the device.
+//
+// It is paid once per lhs, by the first solve.  All on the host it took 1.6 ms
+// for the 9,261 rows of the 20^3 cube and 42 ms for the 517,888 of the CEP slab,
+// mostly the columns of every step and their upload (48 MB).
 #include <algorithm>
 #include <atomic>
 #include <cmath>
@@ -10,19 +15,17 @@
 
 namespace gsls {
 
-// f(b, scratch) for every block b, on up to 8 host threads; the result of a
-// block depends on b only, and it leaves the n scratch entries at -1.  False
-// when host memory could not be had.
+// f(b) for every block b, on up to 8 host threads; the result of a block depends
+// on b only.  False when host memory could not be had.
 template <class F>
-static bool for_blocks(int nblk, long long work, size_t n, const F &f) {
+static bool for_blocks(int nblk, long long work, const F &f) {
   const unsigned hw = std::thread::hardware_concurrency();
   const int T = (int)std::min<long long>(std::min({nblk, 8, hw ? (int)hw : 1}), 1 + work / 40000);
   std::atomic<int> next{0};
   std::atomic<bool> ok{true};
   const auto run = [&] {
     try {
-      std::vector<int> scratch(n, -1);
-      for (int b; (b = next.fetch_add(1)) < nblk;) f(b, scratch);
+      for (int b; (b = next.fetch_add(1)) < nblk;) f(b);
     } catch (...) {
       ok = false;
     }
@@ -38,12 +41,12 @@ static bool for_blocks(int nblk, long long work, size_t n, const F &f) {
   return ok;
 }
 
+// The rows of each block in slot order, their slices and steps
 struct PartHost {
-  int nblk = 0, L = 1, winMax = 0, nslMax = 0, stMax = 0, grpMax = 0;
+  int nblk = 0, L = 1, nslMax = 0, stMax = 0, grpMax = 0;
   long long steps8 = 0;
   bool ok = false;
-  std::vector<int> wbase, sst, soff, sbase, slen, hoff, halo, slotRow, src;
-  std::vector<unsigned short> lcol;
+  std::vector<int> wbase, sst, soff, sbase, slen, slotRow;
 };
 
 static void part_host(int nNo, const std::vector<int> &rp, const std::vector<int> &cp, int sms,
@@ -113,8 +116,10 @@ static void part_host(int nNo, const std::vector<int> &rp, const std::vector<int
       sb[k] = (int)((long long)nblk * k / S);
       sr[k] = k < S ? row0[sb[k]] : nNo;
     }
-    ran = for_blocks(S, rp[nNo], (size_t)nNo, [&](int k, std::vector<int> &seen) {
+    ran = for_blocks(S, rp[nNo], [&](int k) {
       const int r0 = sr[k], r1 = sr[k + 1];
+      std::vector<signed char> mark((size_t)(r1 - r0), -1);  // last pass that saw a row
+      const auto seen = [&](int i) -> signed char & { return mark[i - r0]; };
       int *const o = order.data() + r0;
       int start = r0;
       for (int pass = 0; pass < 2; pass++) {
@@ -124,48 +129,49 @@ static void part_host(int nNo, const std::vector<int> &rp, const std::vector<int
           int at = n;
           if (n == 0 && start < r1) {
             o[n++] = start;
-            seen[start] = pass;
+            seen(start) = (signed char)pass;
           } else {
-            while (seen[next] == pass) next++;
+            while (seen(next) == pass) next++;
             o[n++] = next;
-            seen[next] = pass;
+            seen(next) = (signed char)pass;
           }
           for (; at < n; at++)
             for (int j = rp[o[at]]; j < rp[o[at] + 1]; j++) {
               const int c = cp[j];
-              if (c >= r0 && c < r1 && seen[c] != pass) {
-                seen[c] = pass;
+              if (c >= r0 && c < r1 && seen(c) != pass) {
+                seen(c) = (signed char)pass;
                 o[n++] = c;
               }
             }
         }
         if (n > 0) start = o[n - 1];
       }
-      for (int i = r0; i < r1; i++) seen[i] = -1;
       cut(r0, r1, sb[k], sb[k + 1]);
     });
     if (!ran) throw std::bad_alloc();
   }
-  // pass 1: rows of each block by decreasing length, slices and their steps
+  // rows of each block by decreasing length, then number: slices and their steps
   std::vector<int> &sbase = H.sbase, &slotRow = H.slotRow, &slen = H.slen;
   sbase.assign((size_t)nblk + 1, 0);
-  for (int b = 0; b < nblk; b++) sbase[b + 1] = sbase[b] + (row0[b + 1] - row0[b] + RW - 1) / RW;
+  for (int b = 0; b < nblk; b++) {
+    sbase[b + 1] = sbase[b] + (row0[b + 1] - row0[b] + RW - 1) / RW;
+    H.nslMax = std::max(H.nslMax, sbase[b + 1] - sbase[b]);
+  }
   const int nS = sbase[nblk];
   slotRow.assign((size_t)nS * RW, -1);
   slen.assign(nS, 1);
-  std::vector<int> rowSlot(nNo), blk(nNo);
   std::vector<int> wst((size_t)nblk * W, 0);
-  ran = for_blocks(nblk, rp[nNo], 0, [&](int b, std::vector<int> &) {
+  ran = for_blocks(nblk, nNo, [&](int b) {
     const int r0 = row0[b], r1 = row0[b + 1];
-    std::vector<int> idx(order.begin() + r0, order.begin() + r1);
-    std::sort(idx.begin(), idx.end());
-    std::stable_sort(idx.begin(), idx.end(),
-                     [&](int x, int y) { return rp[x + 1] - rp[x] > rp[y + 1] - rp[y]; });
-    for (int k = 0; k < r1 - r0; k++) {
-      slotRow[(size_t)sbase[b] * RW + k] = idx[k];
-      rowSlot[idx[k]] = sbase[b] * RW + k;
-      blk[idx[k]] = b;
-    }
+    int *const o = order.data() + r0;
+    if (q > 1) std::sort(o, o + (r1 - r0));
+    int longest = 0;
+    for (int k = 0; k < r1 - r0; k++) longest = std::max(longest, rp[o[k] + 1] - rp[o[k]]);
+    std::vector<int> at((size_t)longest + 2, 0);  // first place of each length, longest first
+    for (int k = 0; k < r1 - r0; k++) at[longest - (rp[o[k] + 1] - rp[o[k]]) + 1]++;
+    for (int l = 0; l < longest; l++) at[l + 1] += at[l];
+    for (int k = 0; k < r1 - r0; k++)
+      slotRow[(size_t)sbase[b] * RW + at[longest - (rp[o[k] + 1] - rp[o[k]])]++] = o[k];
     for (int s = sbase[b]; s < sbase[b + 1]; s++) {
       const int i = slotRow[(size_t)s * RW];  // the slice's longest row
       slen[s] = std::max(1, (rp[i + 1] - rp[i] + L - 1) / L);
@@ -183,87 +189,121 @@ static void part_host(int nNo, const std::vector<int> &rp, const std::vector<int
     if (steps > (1LL << 31) / 32 - 1) return;
   }
   wbase[wst.size()] = (int)steps;
-  // slices in steps of their own, from multiples of 8
+  // slices: their first steps in their warp's order, and in steps of their own
+  // from multiples of 8
   H.sst.assign(nS, 0);
   H.soff.assign((size_t)nS + 1, 0);
   long long steps8 = 0;
   std::vector<int> wgr((size_t)nblk * W, 0);
-  for (int b = 0; b < nblk; b++)
+  for (int b = 0; b < nblk; b++) {
+    int next[W];
+    for (int w = 0; w < W; w++) next[w] = wbase[(size_t)b * W + w];
     for (int s = sbase[b]; s < sbase[b + 1]; s++) {
-      const int g = (slen[s] + 7) / 8;
+      const int w = (s - sbase[b]) % W, g = (slen[s] + 7) / 8;
+      H.sst[s] = next[w];
+      next[w] += slen[s];
       H.soff[s] = (int)steps8;
       steps8 += 8 * g;
-      wgr[(size_t)b * W + (s - sbase[b]) % W] += g;
+      wgr[(size_t)b * W + w] += g;
       if (steps8 > (1LL << 31) / 32 - 1 || steps8 - H.soff[sbase[b]] > kGrpOff) return;
     }
+  }
   H.soff[nS] = (int)steps8;
   H.steps8 = steps8;
   for (int g : wgr) H.grpMax = std::max(H.grpMax, g);
-  // pass 2: halo of each block, sources and window columns of its steps
-  std::vector<std::vector<int>> hl(nblk);
-  std::vector<int> &src = H.src;
-  std::vector<unsigned short> &lcol = H.lcol;
-  src.assign((size_t)steps * 32, -1);
-  lcol.assign((size_t)steps * 32, 0);
-  std::vector<char> fit(nblk, 1);
-  ran = for_blocks(nblk, rp[nNo], (size_t)nNo, [&](int b, std::vector<int> &loc) {
-    const int r0 = row0[b], r1 = row0[b + 1], own = (sbase[b + 1] - sbase[b]) * RW;
-    std::vector<int> &h = hl[b];
-    for (int k = r0; k < r1; k++)
-      for (int j = rp[order[k]]; j < rp[order[k] + 1]; j++)
-        if (blk[cp[j]] != b && loc[cp[j]] < 0) {
-          loc[cp[j]] = 0;
-          h.push_back(cp[j]);
-        }
-    std::sort(h.begin(), h.end());
-    if ((long long)own + (long long)h.size() > 65535) {
-      fit[b] = 0;
-      for (int c : h) loc[c] = -1;
-      return;
+  H.ok = true;
+}
+
+// ---- the halos and the steps' columns, on the device
+struct PartBuild {
+  const int *rowPtr, *colPtr, *sbase, *slen, *sst, *slotRow;
+  int *rowSlot;  // slot of each row
+  // per block and 32 nodes: which of them are in its halo, and how many of
+  // its halo's nodes come before
+  uint2 *words;
+  int *count;  // halo entries of each block
+  int nw, L;
+  const int *hoff;
+  int *halo, *src;
+  unsigned short *lcol;
+};
+constexpr int kBuildThreads = 512;
+
+__global__ void k_part_slots(long long n, const int *__restrict__ slotRow, int *rowSlot) {
+  for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < n;
+       k += (long long)gridDim.x * blockDim.x) {
+    const int row = slotRow[k];
+    if (row >= 0) rowSlot[row] = (int)k;
+  }
+}
+
+// halo of block blockIdx.x: 8 lanes per row set the bits of its columns that
+// are not the block's own
+__global__ void __launch_bounds__(kBuildThreads) k_part_mark(PartBuild B) {
+  __shared__ int sh[32];
+  const int b = blockIdx.x, tid = threadIdx.x, RW = 32 / B.L;
+  const int g0 = B.sbase[b] * RW, own = B.sbase[b + 1] * RW - g0;
+  uint2 *w = B.words + (size_t)b * B.nw;
+  for (int k = tid; k < B.nw; k += kBuildThreads) w[k] = make_uint2(0u, 0u);
+  __syncthreads();
+  for (int k = tid >> 3; k < own; k += kBuildThreads >> 3) {
+    const int row = __ldg(B.slotRow + g0 + k);
+    if (row < 0) continue;
+    const int e = __ldg(B.rowPtr + row + 1);
+    for (int j = __ldg(B.rowPtr + row) + (tid & 7); j < e; j += 8) {
+      const int c = __ldg(B.colPtr + j);
+      if ((unsigned)(__ldg(B.rowSlot + c) - g0) < (unsigned)own) continue;
+      const unsigned m = 1u << (c & 31);
+      unsigned *x = &w[c >> 5].x;
+      if (!(*(volatile unsigned *)x & m)) atomicOr(x, m);
     }
-    for (size_t k = 0; k < h.size(); k++) loc[h[k]] = own + (int)k;
-    std::vector<int> at(W);
-    for (int w = 0; w < W; w++) at[w] = wbase[(size_t)b * W + w];
-    for (int s = sbase[b]; s < sbase[b + 1]; s++) {
-      const int w = (s - sbase[b]) % W, st0 = at[w];
-      at[w] += slen[s];
-      H.sst[s] = st0;
-      for (int g = 0; g < RW; g++) {
-        const int i = slotRow[(size_t)s * RW + g];
-        const unsigned short me = (unsigned short)((s - sbase[b]) * RW + g);
-        const int j0 = i >= 0 ? rp[i] : 0, len = i >= 0 ? rp[i + 1] - j0 : 0;
-        for (int t = 0; t < slen[s] * L; t++) {
-          const size_t P = (size_t)(st0 + t / L) * 32 + g * L + t % L;
-          if (t >= len) {
-            lcol[P] = me;  // padding: zero block on the row's own entry
-            continue;
-          }
-          const int c = cp[j0 + t];
-          src[P] = j0 + t;
-          if (blk[c] == b)
-            lcol[P] = (unsigned short)(rowSlot[c] - sbase[b] * RW);
-          else
-            lcol[P] = (unsigned short)loc[c];
+  }
+  __syncthreads();
+  int run = 0;
+  for (int k0 = 0; k0 < B.nw; k0 += kBuildThreads) {
+    const int k = k0 + tid;
+    int tot;
+    const int n = k < B.nw ? __popc(*(volatile unsigned *)&w[k].x) : 0;
+    const int ex = block_scan_excl(n, sh, tot);
+    if (k < B.nw) w[k].y = (unsigned)(run + ex);
+    run += tot;
+    __syncthreads();
+  }
+  if (tid == 0) B.count[b] = run;
+}
+
+// halo (by node number) and, a warp per slice, sources and window columns
+__global__ void __launch_bounds__(kBuildThreads) k_part_fill(PartBuild B) {
+  const int b = blockIdx.x, tid = threadIdx.x, lane = tid & 31, RW = 32 / B.L;
+  const int s0 = B.sbase[b], g0 = s0 * RW, own = B.sbase[b + 1] * RW - g0;
+  const uint2 *__restrict__ w = B.words + (size_t)b * B.nw;
+  for (int k = tid; k < B.nw; k += kBuildThreads) {
+    const uint2 v = w[k];
+    int *out = B.halo + B.hoff[b] + v.y;
+    for (unsigned m = v.x; m; m &= m - 1) *out++ = __ldg(B.rowSlot + 32 * k + __ffs(m) - 1);
+  }
+  const int g = lane / B.L, l = lane - g * B.L;
+  for (int s = tid >> 5; s < own / RW; s += kBuildThreads >> 5) {
+    const int me = s * RW + g, row = __ldg(B.slotRow + g0 + me), len = __ldg(B.slen + s0 + s);
+    const int j0 = row >= 0 ? __ldg(B.rowPtr + row) : 0;
+    const int n = row >= 0 ? __ldg(B.rowPtr + row + 1) - j0 : 0;
+    const size_t P = (size_t)__ldg(B.sst + s0 + s) * 32 + lane;
+#pragma unroll 4
+    for (int t = 0; t < len; t++) {
+      int src = -1, c = me;  // padding: zero block on the row's own entry
+      if (t * B.L + l < n) {
+        src = j0 + t * B.L + l;
+        const int node = __ldg(B.colPtr + src);
+        c = __ldg(B.rowSlot + node) - g0;
+        if ((unsigned)c >= (unsigned)own) {
+          const uint2 v = w[node >> 5];
+          c = own + (int)v.y + __popc(v.x & ((1u << (node & 31)) - 1u));
         }
       }
+      B.src[P + (size_t)t * 32] = src;
+      B.lcol[P + (size_t)t * 32] = (unsigned short)c;
     }
-    for (int &c : h) {
-      loc[c] = -1;
-      c = rowSlot[c];
-    }
-  });
-  if (!ran) throw std::bad_alloc();
-  H.ok = true;
-  H.hoff.assign((size_t)nblk + 1, 0);
-  for (int b = 0; b < nblk; b++) {
-    H.ok = H.ok && fit[b];
-    H.hoff[b + 1] = H.hoff[b] + (int)hl[b].size();
-    H.winMax = std::max(H.winMax, (sbase[b + 1] - sbase[b]) * RW + (int)hl[b].size());
-    H.nslMax = std::max(H.nslMax, sbase[b + 1] - sbase[b]);
   }
-  if (!H.ok) return;
-  H.halo.reserve((size_t)H.hoff[nblk]);
-  for (int b = 0; b < nblk; b++) H.halo.insert(H.halo.end(), hl[b].begin(), hl[b].end());
 }
 
 // v appended to the image of the device buffer at a 16-byte boundary; its offset
@@ -275,74 +315,136 @@ static size_t append(std::vector<unsigned char> &img, const std::vector<T> &v) {
   return at;
 }
 
-static int part_build(gsls_lhs *lhs, RowPart &p) {
-  PartHost H;
-  part_host(lhs->nNo, lhs->h_rowPtr, lhs->h_colPtr, num_sms(), H);
-  p.ok = H.ok;
-  if (H.ok) {
-    std::vector<unsigned char> img;
-    img.reserve(sizeof(int) * (H.wbase.size() + 2 * H.soff.size() + H.sbase.size() + H.slen.size() + H.hoff.size() +
-                               H.halo.size() + H.slotRow.size() + H.src.size()) +
-                2 * H.lcol.size() + 256);
-    p.off[0] = append(img, H.wbase);
-    p.off[1] = append(img, H.sbase);
-    p.off[2] = append(img, H.slen);
-    p.off[3] = append(img, H.hoff);
-    p.off[4] = append(img, H.halo);
-    p.off[5] = append(img, H.slotRow);
-    p.off[6] = append(img, H.src);
-    p.off[7] = append(img, H.lcol);
-    p.off[8] = append(img, H.sst);
-    p.off[9] = append(img, H.soff);
-    if (!p.buf.try_alloc(img.size() + 16)) {
-      p.ok = false;
-      p.built = true;
-      return GSLS_OK;
-    }
-    GSLS_CUDA(cudaMemcpyAsync(p.buf.p, img.data(), img.size(), cudaMemcpyHostToDevice,
-                              lhs->stream));
-    GSLS_CUDA(cudaStreamSynchronize(lhs->stream));  // img goes out of scope
-    p.L = H.L;
-    p.winMax = H.winMax;
-    p.nslMax = H.nslMax;
-    p.stMax = H.stMax;
-    p.grpMax = H.grpMax;
-    p.nS = (int)H.slen.size();
-    p.steps8 = H.steps8;
-    p.slots = (long long)H.slotRow.size();
-    p.steps = (long long)H.wbase.back();
-  }
-  p.nblk = H.nblk;
-  p.built = true;
+static PartBuild part_build(const gsls_lhs *lhs, const RowPart &p) {
+  const PartArgs a = part_args(p);
+  PartBuild B{};
+  B.rowPtr = lhs->d_rowPtr.as<int>();
+  B.colPtr = lhs->d_colPtr.as<int>();
+  B.sbase = a.sbase;
+  B.slen = a.slen;
+  B.sst = a.sst;
+  B.slotRow = a.slotRow;
+  B.nw = (lhs->nNo + 31) / 32;
+  B.L = p.L;
+  B.words = p.tmp.as<uint2>();
+  B.rowSlot = reinterpret_cast<int *>(B.words + (size_t)B.nw * p.nblk);
+  B.count = B.rowSlot + lhs->nNo;
+  return B;
+}
+
+// the halos as bits in p.tmp; *ok false when there is no memory for them
+static int part_mark(gsls_lhs *lhs, RowPart &p, bool *ok) {
+  const size_t nw = ((size_t)lhs->nNo + 31) / 32;
+  *ok = p.tmp.try_alloc(nw * p.nblk * sizeof(uint2) + sizeof(int) * ((size_t)lhs->nNo + p.nblk));
+  if (!*ok) return GSLS_OK;
+  const PartBuild B = part_build(lhs, p);
+  k_part_slots<<<4 * num_sms(), 256, 0, lhs->stream>>>(p.slots, B.slotRow, B.rowSlot);
+  GSLS_CHECK_LAUNCH();
+  k_part_mark<<<p.nblk, kBuildThreads, 0, lhs->stream>>>(B);
+  GSLS_CHECK_LAUNCH();
   return GSLS_OK;
 }
 
 int part_setup(gsls_lhs *lhs) {
   RowPart &p = lhs->ws.part;
   if (p.built) return GSLS_OK;
+  p.built = true;
+  cudaStream_t st = lhs->stream;
+  PartHost H;
+  std::vector<unsigned char> img;
   try {
-    return part_build(lhs, p);
+    part_host(lhs->nNo, lhs->h_rowPtr, lhs->h_colPtr, num_sms(), H);
+    if (!H.ok) return GSLS_OK;
+    p.hoff.assign((size_t)H.nblk + 1, 0);
+    img.reserve(sizeof(int) * (H.wbase.size() + 2 * H.soff.size() + 2 * H.sbase.size() +
+                               H.slen.size() + H.slotRow.size()) + 256);
+    p.off[0] = append(img, H.wbase);
+    p.off[1] = append(img, H.sbase);
+    p.off[2] = append(img, H.slen);
+    p.off[3] = append(img, p.hoff);
+    p.off[4] = append(img, H.slotRow);
+    p.off[5] = append(img, H.sst);
+    p.off[6] = append(img, H.soff);
   } catch (const std::bad_alloc &) {
-    p.ok = false;
-    p.built = true;
     return GSLS_OK;
   }
+  if (!p.buf.try_alloc(img.size() + 16)) return GSLS_OK;
+  GSLS_CUDA(cudaMemcpyAsync(p.buf.p, img.data(), img.size(), cudaMemcpyHostToDevice, st));
+  p.L = H.L;
+  p.nslMax = H.nslMax;
+  p.stMax = H.stMax;
+  p.grpMax = H.grpMax;
+  p.nS = (int)H.slen.size();
+  p.steps8 = H.steps8;
+  p.slots = (long long)H.slotRow.size();
+  p.steps = (long long)H.wbase.back();
+  p.nblk = H.nblk;
+  bool ok;
+  GSLS_TRY(part_mark(lhs, p, &ok));
+  if (ok)
+    GSLS_CUDA(cudaMemcpyAsync(p.hoff.data() + 1, part_build(lhs, p).count,
+                              sizeof(int) * (size_t)p.nblk, cudaMemcpyDeviceToHost, st));
+  GSLS_CUDA(cudaStreamSynchronize(st));  // also: img goes out of scope
+  for (int b = 0; ok && b < p.nblk; b++) {
+    const long long win = (long long)(H.sbase[b + 1] - H.sbase[b]) * (32 / p.L) + p.hoff[b + 1];
+    ok = win <= 65535;  // 16-bit columns; bounds the sum of the halos too
+    if (!ok) break;
+    p.winMax = std::max(p.winMax, (int)win);
+    p.hoff[b + 1] += p.hoff[b];
+  }
+  if (!ok) {
+    p.buf.release();
+    p.tmp.release();
+    return GSLS_OK;
+  }
+  GSLS_CUDA(cudaMemcpyAsync(p.buf.as<unsigned char>() + p.off[3], p.hoff.data(),
+                            sizeof(int) * p.hoff.size(), cudaMemcpyHostToDevice, st));
+  p.ok = true;
+  return GSLS_OK;
+}
+
+int part_fill(gsls_lhs *lhs) {
+  RowPart &p = lhs->ws.part;
+  if (p.tab.p) return GSLS_OK;
+  const size_t nh = (size_t)p.hoff[p.nblk], n = (size_t)p.steps * 32;
+  bool ok = p.tab.try_alloc(sizeof(int) * (nh + n) + sizeof(short) * n + 16);
+  if (ok && !p.tmp.p) GSLS_TRY(part_mark(lhs, p, &ok));
+  if (!ok) {
+    p.ok = false;
+    p.tab.release();
+    p.buf.release();
+    p.tmp.release();
+    return GSLS_OK;
+  }
+  const PartArgs a = part_args(p);
+  PartBuild B = part_build(lhs, p);
+  B.hoff = a.hoff;
+  B.halo = const_cast<int *>(a.halo);
+  B.src = const_cast<int *>(a.src);
+  B.lcol = const_cast<unsigned short *>(a.lcol);
+  k_part_fill<<<p.nblk, kBuildThreads, 0, lhs->stream>>>(B);
+  GSLS_CHECK_LAUNCH();
+  GSLS_CUDA(cudaStreamSynchronize(lhs->stream));
+  p.tmp.release();
+  return GSLS_OK;
 }
 
 PartArgs part_args(const RowPart &p) {
-  PartArgs a;
+  PartArgs a{};
   const unsigned char *d = p.buf.as<unsigned char>();
   const auto ints = [&](int k) { return reinterpret_cast<const int *>(d + p.off[k]); };
   a.wbase = ints(0);
   a.sbase = ints(1);
   a.slen = ints(2);
   a.hoff = ints(3);
-  a.halo = ints(4);
-  a.slotRow = ints(5);
-  a.src = ints(6);
-  a.sst = ints(8);
-  a.soff = ints(9);
-  a.lcol = reinterpret_cast<const unsigned short *>(d + p.off[7]);
+  a.slotRow = ints(4);
+  a.sst = ints(5);
+  a.soff = ints(6);
+  a.halo = p.tab.as<int>();
+  if (a.halo) {
+    a.src = a.halo + p.hoff[p.nblk];
+    a.lcol = reinterpret_cast<const unsigned short *>(a.src + (size_t)p.steps * 32);
+  }
   a.nblk = p.nblk;
   a.L = p.L;
   a.winMax = p.winMax;

@@ -43,11 +43,19 @@ struct PartArgs {
   long long nslots, nsteps, nsteps8;  // slots; steps, and those of soff
 };
 
-// Partition of the lhs over at most num_sms() blocks; built on the host once
-// per lhs.  ok is false when a window has more than 65,535 entries or there is
-// no memory for the tables: the callers then have kernels without them.
+// Partition of the lhs over at most num_sms() blocks, once per lhs: part_setup
+// orders the rows and sizes the windows, part_fill makes the tables of the
+// halos and steps for a caller whose windows fit.  ok is false when a window
+// has more than 65,535 entries or there is no memory for the tables: the
+// callers then have kernels without them.
 int part_setup(gsls_lhs *lhs);
+int part_fill(gsls_lhs *lhs);
 PartArgs part_args(const RowPart &p);
+// least rows of the largest block: where these alone do not fit, nothing is built
+inline long long part_rows(const gsls_lhs *lhs) {
+  const long long nblk = num_sms() < kPartMaxBlocks ? num_sms() : kPartMaxBlocks;
+  return (lhs->nNo + nblk - 1) / nblk;
+}
 
 // Most dynamic shared memory of a block of the kernel on this device
 inline size_t smem_cap(const void *kernel) {

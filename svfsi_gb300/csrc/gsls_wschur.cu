@@ -362,9 +362,16 @@ template <class VT>
 int wschur_pack(gsls_lhs *lhs, const VT *mG, const VT *Gt, const VT *mL, bool *fits) {
   *fits = false;
   Workspace &ws = lhs->ws;
+  // P and GP of the own rows, X, R and SP
+  if (part_rows(lhs) * 7 * (long long)sizeof(VT) > (long long)wschur_cap<VT, VT>()) return GSLS_OK;
   GSLS_TRY(part_setup(lhs));
   if (!ws.part.ok) return GSLS_OK;
-  if (wschur_smem<VT>(ws.part) > wschur_cap<VT, VT>()) return GSLS_OK;
+  if (wschur_smem<VT>(ws.part) > wschur_cap<VT, VT>()) {
+    ws.part.tmp.release();
+    return GSLS_OK;
+  }
+  GSLS_TRY(part_fill(lhs));
+  if (!ws.part.ok) return GSLS_OK;
   const PartArgs P = part_args(ws.part);
   const size_t n1 = (size_t)P.nsteps8 * SRec<3, VT>::SB, n2 = (size_t)P.nsteps8 * SRec<4, VT>::SB;
   const size_t vb = ((size_t)P.nslots * sizeof(VT) + 127) & ~(size_t)127;
