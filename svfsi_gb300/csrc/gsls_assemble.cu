@@ -36,7 +36,8 @@ struct gsls_mesh {
   // element blocks of each CSR block (gsls_asm_gather.cuh), one map per window
   // of kInvEl elements, and the element buffer
   struct Inverse {
-    gsls::DevBuf ptr, ent;
+    gsls::DevBuf buf;
+    int *ptr, *ent;
   };
   std::vector<std::unique_ptr<Inverse>> inv;
   gsls::DevBuf d_el;
@@ -494,40 +495,44 @@ static int asm_launch(K kern, int nb, cudaStream_t st, const AsmArgs &A, bool pd
   return GSLS_OK;
 }
 
-// inverse element -> CSR map, on the first gathered assembly of a mesh
+// inverse element -> CSR map, on the first gathered assembly of a mesh; its
+// counters live in the element buffer, which is not in use yet (allocations and
+// frees of their own made that assembly 0.1 ms longer than the colour launches)
 static int inv_prepare(gsls_mesh *m) {
   if (m->inv_ready) return GSLS_OK;
   gsls_lhs *lhs = m->lhs;
   cudaStream_t st = lhs->stream;
   const int nnz = lhs->nnz, nb = (nnz + kScan - 1) / kScan, g = 8 * num_sms();
-  DevBuf cnt, sums;
-  GSLS_TRY(cnt.alloc(sizeof(int) * (size_t)nnz));
-  GSLS_TRY(sums.alloc(sizeof(int) * (size_t)nb));
+  const size_t need = sizeof(int) * ((size_t)nnz + nb);
+  DevBuf own;
+  if (need > m->d_el.bytes) GSLS_TRY(own.alloc(need));
+  int *cnt = own.p ? own.as<int>() : m->d_el.as<int>(), *sums = cnt + nnz;
   const size_t nw = ((size_t)m->nEl + kInvEl - 1) / kInvEl;
   m->inv.clear();
   for (size_t w = 0; w < nw; w++) {
     m->inv.emplace_back(new gsls_mesh::Inverse);
     gsls_mesh::Inverse &v = *m->inv.back();
     const size_t n = 16 * std::min<size_t>(kInvEl, (size_t)m->nEl - w * kInvEl);
-    GSLS_TRY(v.ptr.alloc(sizeof(int) * ((size_t)nnz + 1)));
-    GSLS_TRY(v.ent.alloc(sizeof(int) * n));
+    GSLS_TRY(v.buf.alloc(sizeof(int) * ((size_t)nnz + 1 + n)));
+    v.ptr = v.buf.as<int>();
+    v.ent = v.ptr + nnz + 1;
     const int *map = m->d_map.as<int>() + 16 * kInvEl * w;
-    int *ptr = v.ptr.as<int>(), *ent = v.ent.as<int>();
-    GSLS_CUDA(cudaMemsetAsync(cnt.p, 0, sizeof(int) * (size_t)nnz, st));
-    k_inv_count<<<g, 256, 0, st>>>(n, map, cnt.as<int>());
+    int *ptr = v.ptr, *ent = v.ent;
+    GSLS_CUDA(cudaMemsetAsync(cnt, 0, sizeof(int) * (size_t)nnz, st));
+    k_inv_count<<<g, 256, 0, st>>>(n, map, cnt);
     GSLS_CHECK_LAUNCH();
-    k_scan_sums<<<nb, 256, 0, st>>>(nnz, cnt.as<int>(), sums.as<int>());
+    k_scan_sums<<<nb, 256, 0, st>>>(nnz, cnt, sums);
     GSLS_CHECK_LAUNCH();
-    k_scan_top<<<1, 1024, 0, st>>>(nb, sums.as<int>());
+    k_scan_top<<<1, 1024, 0, st>>>(nb, sums);
     GSLS_CHECK_LAUNCH();
-    k_scan_fill<<<nb, 256, 0, st>>>(nnz, cnt.as<int>(), sums.as<int>(), ptr, (int)n);
+    k_scan_fill<<<nb, 256, 0, st>>>(nnz, cnt, sums, ptr, (int)n);
     GSLS_CHECK_LAUNCH();
-    k_inv_fill<<<g, 256, 0, st>>>(n, map, ptr, cnt.as<int>(), ent);
+    k_inv_fill<<<g, 256, 0, st>>>(n, map, ptr, cnt, ent);
     GSLS_CHECK_LAUNCH();
     k_inv_sort<<<g, 256, 0, st>>>(nnz, ptr, ent);
     GSLS_CHECK_LAUNCH();
   }
-  GSLS_CUDA(cudaStreamSynchronize(st));  // cnt and sums go out of scope
+  if (own.p) GSLS_CUDA(cudaStreamSynchronize(st));  // it goes out of scope
   m->inv_ready = true;
   return GSLS_OK;
 }
@@ -537,7 +542,6 @@ static int inv_prepare(gsls_mesh *m) {
 template <int DOF, class VT, class K>
 static int assemble_gather(gsls_mesh *m, K kern, size_t smem, AsmArgs A, double *R, VT *Val) {
   std::lock_guard<std::mutex> lk(m->el_mu);
-  GSLS_TRY(inv_prepare(m));
   constexpr int DD = DOF * DOF;
   gsls_lhs *lhs = m->lhs;
   cudaStream_t st = lhs->stream;
@@ -558,6 +562,7 @@ static int assemble_gather(gsls_mesh *m, K kern, size_t smem, AsmArgs A, double 
     n = std::max(n / 2, (size_t)4096 * per);
     m->el_most = n;
   }
+  GSLS_TRY(inv_prepare(m));
   const int part = (int)std::min<size_t>((size_t)m->nEl, m->d_el.bytes / per);
   A.lK = m->d_el.p;
   A.lR = reinterpret_cast<double *>(m->d_el.as<unsigned char>() + kEl * (size_t)part);
@@ -568,7 +573,7 @@ static int assemble_gather(gsls_mesh *m, K kern, size_t smem, AsmArgs A, double 
     // elements of this part, all in one window of the inverse map
     const int w = e0 / kInvEl, f = e0 - w * kInvEl;
     ne = std::min(std::min(part, m->nEl - e0), kInvEl - f);
-    const int *ptr = m->inv[w]->ptr.as<int>(), *ent = m->inv[w]->ent.as<int>();
+    const int *ptr = m->inv[w]->ptr, *ent = m->inv[w]->ent;
     A.el0 = e0;
     A.nColorEl = ne;
     kern<<<(ne + kAsmThreads - 1) / kAsmThreads, kAsmThreads, sm, st>>>(A);
