@@ -15,12 +15,12 @@
 
 namespace gsls {
 
-// f(b) for every block b, on up to 8 host threads; the result of a block depends
+// f(b) for every block b, on up to 16 host threads; the result of a block depends
 // on b only.  False when host memory could not be had.
 template <class F>
 static bool for_blocks(int nblk, long long work, const F &f) {
   const unsigned hw = std::thread::hardware_concurrency();
-  const int T = (int)std::min<long long>(std::min({nblk, 8, hw ? (int)hw : 1}), 1 + work / 40000);
+  const int T = (int)std::min<long long>(std::min({nblk, 16, hw ? (int)hw : 1}), 1 + work / 40000);
   std::atomic<int> next{0};
   std::atomic<bool> ok{true};
   const auto run = [&] {
