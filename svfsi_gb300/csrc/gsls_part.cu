@@ -147,6 +147,12 @@ static void part_host(int nNo, const std::vector<int> &rp, const std::vector<int
         if (n > 0) start = o[n - 1];
       }
       cut(r0, r1, sb[k], sb[k + 1]);
+      // the rows of each block by number; at most nblk / S + 1 < 128 blocks
+      std::vector<int> at(row0.begin() + sb[k], row0.begin() + sb[k + 1]);
+      for (int b = sb[k]; b < sb[k + 1]; b++)
+        for (int i = row0[b]; i < (b + 1 < sb[k + 1] ? row0[b + 1] : r1); i++)
+          seen(order[i]) = (signed char)(b - sb[k]);
+      for (int i = r0; i < r1; i++) order[at[seen(i)]++] = i;
     });
     if (!ran) throw std::bad_alloc();
   }
@@ -164,7 +170,6 @@ static void part_host(int nNo, const std::vector<int> &rp, const std::vector<int
   ran = for_blocks(nblk, nNo, [&](int b) {
     const int r0 = row0[b], r1 = row0[b + 1];
     int *const o = order.data() + r0;
-    if (q > 1) std::sort(o, o + (r1 - r0));
     int longest = 0;
     for (int k = 0; k < r1 - r0; k++) longest = std::max(longest, rp[o[k] + 1] - rp[o[k]]);
     std::vector<int> at((size_t)longest + 2, 0);  // first place of each length, longest first
