@@ -99,6 +99,7 @@ static_assert(sizeof(KrylovScalars) <= kScalRed, "scalar block");
 // Row partition of the persistent kernels (gsls_part.cuh)
 struct RowPart {
   bool built = false, ok = false;
+  bool scattered = false;  // halos many times those of compact blocks
   int nblk = 0, L = 1, winMax = 0, nslMax = 0, stMax = 0, grpMax = 0, nS = 0;
   long long slots = 0, steps = 0, steps8 = 0;
   DevBuf buf;             // the tables per slot, slice and block, at their offsets
@@ -168,7 +169,8 @@ struct Workspace {
   long long sell_steps = 0;
   DevBuf sell_off, sell_row, sell_col, sell_pos, sell_val;
   // row partition; stream and vectors of the windowed CG (gsls_wcg.cu)
-  RowPart part;
+  RowPart part[2];
+  RowPart *ns_part = nullptr;  // the one that ns_stream is laid out on
   DevBuf wcg_stream, wcg_vec;
   unsigned long long wcg_serial = 0;  // preconditioning whose matrix the stream holds
   const void *wcg_val = nullptr;      // (and the array it was packed from)

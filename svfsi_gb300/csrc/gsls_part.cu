@@ -219,12 +219,52 @@ static void part_host(int nNo, const std::vector<int> &rp, const std::vector<int
   H.ok = true;
 }
 
+// The same on the graph's own numbering: breadth-first from a far end, which is
+// where the search from row 0 ends.  A block of consecutive rows then lies
+// together whatever numbering the mesh came with.
+static void part_host_graph(int nNo, const std::vector<int> &rp, const std::vector<int> &cp,
+                            int sms, PartHost &H) {
+  std::vector<int> row((size_t)nNo), num((size_t)nNo, -1);  // row of a number, number of a row
+  int start = 0;
+  for (int pass = 0; pass < 2; pass++) {
+    std::fill(num.begin(), num.end(), -1);
+    int n = 0, next = 0;
+    while (n < nNo) {
+      int at = n;
+      if (n > 0) {
+        while (num[next] >= 0) next++;
+        start = next;
+      }
+      num[start] = n;
+      row[n++] = start;
+      for (; at < n; at++)
+        for (int j = rp[row[at]]; j < rp[row[at] + 1]; j++)
+          if (num[cp[j]] < 0) {
+            num[cp[j]] = n;
+            row[n++] = cp[j];
+          }
+    }
+    start = row[nNo - 1];
+  }
+  std::vector<int> rpn((size_t)nNo + 1), cpn((size_t)rp[nNo]);
+  for (int i = 0; i < nNo; i++) rpn[i + 1] = rpn[i] + rp[row[i] + 1] - rp[row[i]];
+  const int nb = 64;
+  const bool ran = for_blocks(nb, rp[nNo], [&](int b) {
+    for (int i = (int)((long long)nNo * b / nb); i < (int)((long long)nNo * (b + 1) / nb); i++)
+      for (int j = rp[row[i]], k = rpn[i]; j < rp[row[i] + 1]; j++) cpn[k++] = num[cp[j]];
+  });
+  if (!ran) throw std::bad_alloc();
+  part_host(nNo, rpn, cpn, sms, H);
+  for (int &i : H.slotRow)
+    if (i >= 0) i = row[i];
+}
+
 // ---- the halos and the steps' columns, on the device
 struct PartBuild {
   const int *rowPtr, *colPtr, *sbase, *slen, *sst, *slotRow;
   int *rowSlot;  // slot of each row
-  // per block and 32 nodes: which of them are in its halo, and how many of
-  // its halo's nodes come before
+  // per block and 32 slots: which of them are in its halo, and how many of
+  // its halo's slots come before
   uint2 *words;
   int *count;  // halo entries of each block
   int nw, L;
@@ -256,8 +296,8 @@ __global__ void __launch_bounds__(kBuildThreads) k_part_mark(PartBuild B) {
     if (row < 0) continue;
     const int e = __ldg(B.rowPtr + row + 1);
     for (int j = __ldg(B.rowPtr + row) + (tid & 7); j < e; j += 8) {
-      const int c = __ldg(B.colPtr + j);
-      if ((unsigned)(__ldg(B.rowSlot + c) - g0) < (unsigned)own) continue;
+      const int c = __ldg(B.rowSlot + __ldg(B.colPtr + j));
+      if ((unsigned)(c - g0) < (unsigned)own) continue;
       const unsigned m = 1u << (c & 31);
       unsigned *x = &w[c >> 5].x;
       if (!(*(volatile unsigned *)x & m)) atomicOr(x, m);
@@ -277,7 +317,8 @@ __global__ void __launch_bounds__(kBuildThreads) k_part_mark(PartBuild B) {
   if (tid == 0) B.count[b] = run;
 }
 
-// halo (by node number) and, a warp per slice, sources and window columns
+// halo (by slot: neighbouring entries of it are neighbours in the vectors) and,
+// a warp per slice, sources and window columns
 __global__ void __launch_bounds__(kBuildThreads) k_part_fill(PartBuild B) {
   const int b = blockIdx.x, tid = threadIdx.x, lane = tid & 31, RW = 32 / B.L;
   const int s0 = B.sbase[b], g0 = s0 * RW, own = B.sbase[b + 1] * RW - g0;
@@ -285,7 +326,7 @@ __global__ void __launch_bounds__(kBuildThreads) k_part_fill(PartBuild B) {
   for (int k = tid; k < B.nw; k += kBuildThreads) {
     const uint2 v = w[k];
     int *out = B.halo + B.hoff[b] + v.y;
-    for (unsigned m = v.x; m; m &= m - 1) *out++ = __ldg(B.rowSlot + 32 * k + __ffs(m) - 1);
+    for (unsigned m = v.x; m; m &= m - 1) *out++ = 32 * k + __ffs(m) - 1;
   }
   const int g = lane / B.L, l = lane - g * B.L;
   for (int s = tid >> 5; s < own / RW; s += kBuildThreads >> 5) {
@@ -298,11 +339,11 @@ __global__ void __launch_bounds__(kBuildThreads) k_part_fill(PartBuild B) {
       int src = -1, c = me;  // padding: zero block on the row's own entry
       if (t * B.L + l < n) {
         src = j0 + t * B.L + l;
-        const int node = __ldg(B.colPtr + src);
-        c = __ldg(B.rowSlot + node) - g0;
+        const int slot = __ldg(B.rowSlot + __ldg(B.colPtr + src));
+        c = slot - g0;
         if ((unsigned)c >= (unsigned)own) {
-          const uint2 v = w[node >> 5];
-          c = own + (int)v.y + __popc(v.x & ((1u << (node & 31)) - 1u));
+          const uint2 v = w[slot >> 5];
+          c = own + (int)v.y + __popc(v.x & ((1u << (slot & 31)) - 1u));
         }
       }
       B.src[P + (size_t)t * 32] = src;
@@ -329,7 +370,7 @@ static PartBuild part_build(const gsls_lhs *lhs, const RowPart &p) {
   B.slen = a.slen;
   B.sst = a.sst;
   B.slotRow = a.slotRow;
-  B.nw = (lhs->nNo + 31) / 32;
+  B.nw = (int)((p.slots + 31) / 32);
   B.L = p.L;
   B.words = p.tmp.as<uint2>();
   B.rowSlot = reinterpret_cast<int *>(B.words + (size_t)B.nw * p.nblk);
@@ -339,7 +380,7 @@ static PartBuild part_build(const gsls_lhs *lhs, const RowPart &p) {
 
 // the halos as bits in p.tmp; *ok false when there is no memory for them
 static int part_mark(gsls_lhs *lhs, RowPart &p, bool *ok) {
-  const size_t nw = ((size_t)lhs->nNo + 31) / 32;
+  const size_t nw = ((size_t)p.slots + 31) / 32;
   *ok = p.tmp.try_alloc(nw * p.nblk * sizeof(uint2) + sizeof(int) * ((size_t)lhs->nNo + p.nblk));
   if (!*ok) return GSLS_OK;
   const PartBuild B = part_build(lhs, p);
@@ -350,15 +391,15 @@ static int part_mark(gsls_lhs *lhs, RowPart &p, bool *ok) {
   return GSLS_OK;
 }
 
-int part_setup(gsls_lhs *lhs) {
-  RowPart &p = lhs->ws.part;
+int part_setup(gsls_lhs *lhs, bool graph) {
+  RowPart &p = lhs->ws.part[graph];
   if (p.built) return GSLS_OK;
   p.built = true;
   cudaStream_t st = lhs->stream;
   PartHost H;
   std::vector<unsigned char> img;
   try {
-    part_host(lhs->nNo, lhs->h_rowPtr, lhs->h_colPtr, num_sms(), H);
+    (graph ? part_host_graph : part_host)(lhs->nNo, lhs->h_rowPtr, lhs->h_colPtr, num_sms(), H);
     if (!H.ok) return GSLS_OK;
     p.hoff.assign((size_t)H.nblk + 1, 0);
     img.reserve(sizeof(int) * (H.wbase.size() + 2 * H.soff.size() + 2 * H.sbase.size() +
@@ -390,6 +431,15 @@ int part_setup(gsls_lhs *lhs) {
     GSLS_CUDA(cudaMemcpyAsync(p.hoff.data() + 1, part_build(lhs, p).count,
                               sizeof(int) * (size_t)p.nblk, cudaMemcpyDeviceToHost, st));
   GSLS_CUDA(cudaStreamSynchronize(st));  // also: img goes out of scope
+  if (ok) {
+    // a compact block of r rows has about (r^1/3 + 2)^3 - r neighbours; meshes
+    // numbered plane by plane have up to 3.3 times as many in all (the CEP
+    // slab), the same meshes numbered at random 5 to 13 times
+    double halos = 0.0;
+    const double r = (double)lhs->nNo / p.nblk;
+    for (int b = 0; b < p.nblk; b++) halos += p.hoff[b + 1];
+    p.scattered = halos > 4.0 * p.nblk * (pow(cbrt(r) + 2.0, 3.0) - r);
+  }
   for (int b = 0; ok && b < p.nblk; b++) {
     const long long win = (long long)(H.sbase[b + 1] - H.sbase[b]) * (32 / p.L) + p.hoff[b + 1];
     ok = win <= 65535;  // 16-bit columns; bounds the sum of the halos too
@@ -408,8 +458,7 @@ int part_setup(gsls_lhs *lhs) {
   return GSLS_OK;
 }
 
-int part_fill(gsls_lhs *lhs) {
-  RowPart &p = lhs->ws.part;
+int part_fill(gsls_lhs *lhs, RowPart &p) {
   if (p.tab.p) return GSLS_OK;
   const size_t nh = (size_t)p.hoff[p.nblk], n = (size_t)p.steps * 32;
   bool ok = p.tab.try_alloc(sizeof(int) * (nh + n) + sizeof(short) * n + 16);

@@ -474,17 +474,15 @@ static int wcg_t(gsls_lhs *lhs, gsls_sub_ls *ls, const VT *Val, double *R, const
   // window and KP of the own rows
   if (part_rows(lhs) * 2 * D * (long long)sizeof(XT) > (long long)wcg_cap<D, VT, XT>())
     return GSLS_OK;
-  GSLS_TRY(part_setup(lhs));
-  if (!ws.part.ok) return GSLS_OK;
   WcgArgs<XT> A{};
-  const size_t smem = wcg_geometry<D, VT, XT>(part_args(ws.part), A);
-  if (!smem) {
-    ws.part.tmp.release();
-    return GSLS_OK;
-  }
-  GSLS_TRY(part_fill(lhs));
-  if (!ws.part.ok) return GSLS_OK;
-  const PartArgs P = part_args(ws.part);
+  size_t smem = 0;
+  RowPart *part;
+  GSLS_TRY(part_for(lhs, &part, [&](const RowPart &p) {
+    smem = wcg_geometry<D, VT, XT>(part_args(p), A);
+    return smem != 0;
+  }));
+  if (!part) return GSLS_OK;
+  const PartArgs P = part_args(*part);
   const size_t vb = ((size_t)P.nslots * NodeL2<D, XT>::VD * sizeof(XT) + 127) & ~(size_t)127;
   const size_t sb = Rec<D, VT>::at(P.nsteps, P.nblk * kPartWarps);
   // no memory for a second copy of the matrix: the batched kernels take the

@@ -364,15 +364,11 @@ int wschur_pack(gsls_lhs *lhs, const VT *mG, const VT *Gt, const VT *mL, bool *f
   Workspace &ws = lhs->ws;
   // P and GP of the own rows, X, R and SP
   if (part_rows(lhs) * 7 * (long long)sizeof(VT) > (long long)wschur_cap<VT, VT>()) return GSLS_OK;
-  GSLS_TRY(part_setup(lhs));
-  if (!ws.part.ok) return GSLS_OK;
-  if (wschur_smem<VT>(ws.part) > wschur_cap<VT, VT>()) {
-    ws.part.tmp.release();
-    return GSLS_OK;
-  }
-  GSLS_TRY(part_fill(lhs));
-  if (!ws.part.ok) return GSLS_OK;
-  const PartArgs P = part_args(ws.part);
+  GSLS_TRY(part_for(lhs, &ws.ns_part, [](const RowPart &p) {
+    return wschur_smem<VT>(p) <= wschur_cap<VT, VT>();
+  }));
+  if (!ws.ns_part) return GSLS_OK;
+  const PartArgs P = part_args(*ws.ns_part);
   const size_t n1 = (size_t)P.nsteps8 * SRec<3, VT>::SB, n2 = (size_t)P.nsteps8 * SRec<4, VT>::SB;
   const size_t vb = ((size_t)P.nslots * sizeof(VT) + 127) & ~(size_t)127;
   // no memory for the streams: the per-kernel Schur CG, without another try
@@ -395,13 +391,13 @@ template <class VT, class XT>
 int wschur_run(gsls_lhs *lhs, const gsls_sub_ls *ls, XT *x, SchurScal *out) {
   Workspace &ws = lhs->ws;
   cudaStream_t st = lhs->stream;
-  const PartArgs P = part_args(ws.part);
+  const PartArgs P = part_args(*ws.ns_part);
   const size_t n1 = ((size_t)P.nsteps8 * SRec<3, VT>::SB + 127) & ~(size_t)127;
   const size_t n2 = ((size_t)P.nsteps8 * SRec<4, VT>::SB + 127) & ~(size_t)127;
   const size_t vb = ((size_t)P.nslots * sizeof(XT) + 127) & ~(size_t)127;
   unsigned char *s1 = ws.ns_stream.as<unsigned char>();
   unsigned char *sc = ws.scal.as<unsigned char>();
-  const size_t smem = wschur_smem<XT>(ws.part);
+  const size_t smem = wschur_smem<XT>(*ws.ns_part);
   GSLS_CUDA(cudaMemsetAsync(sc + kScalRed, 0, sizeof(GridBar), st));
   WschurArgs<XT> A{};
   A.P = P;

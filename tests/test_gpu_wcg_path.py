@@ -1,6 +1,7 @@
 """Which kernels a CG solve takes: the one launch on the row partition wherever
 a block's window fits in shared memory, the batched kernels where it does not,
-told apart by the library's profile counters.
+told apart by the library's profile counters.  A mesh numbered at random fits in
+the order of its graph.
 
 The graph that does not fit is random with 80 neighbours per node: a block of
 the 152 (264 rows) sees about 16,000 other nodes, which with 16 bytes each (4
@@ -81,3 +82,25 @@ def test_windows_that_do_not_fit(gsls, orc):
         assert ran == [False, True]
         assert np.linalg.norm(x - Ro) <= 10 * tol * np.linalg.norm(Ro)
         lhs.free()
+
+
+@pytest.mark.parametrize("mixed", [False, True])
+def test_scattered_numbering_takes_the_order_of_the_graph(gsls, orc, mixed):
+    """120 x 100 x 20 hexes numbered at random: windows of 25,000 entries, which
+    do not fit with 3 values each, and of 3,500 in the order of the graph."""
+    torch = pytest.importorskip("torch")
+    rp, cp = _graph(("shuffled", 120, 100, 20))
+    n, d = rp.size - 1, 3
+    own = n // 152
+    seen = np.unique(cp[rp[own * 70]:rp[own * 71]])
+    assert 4 * d * (seen.size + own) > 232448
+    V0, R0 = _system(rp, cp, d, 7)
+    s = orc.OracleSolver(n, rp.astype(np.int32), cp.astype(np.int32), 1)
+    Ro, Vo = R0.copy(), V0.copy()
+    s.solve(orc.ls_create(orc.LS_TYPE_CG, relTol=1e-10, mItr=500), d, Ro, Vo, orc.PRECOND_FSILS)
+    lhs = _lhs(rp, cp)
+    tol = 1e-5 if mixed else 1e-10
+    x, ran = _solve(gsls, torch, lhs, d, R0, V0, mixed, tol, 500)
+    assert ran == [True, False]
+    assert np.linalg.norm(x - Ro) <= 10 * tol * np.linalg.norm(Ro)
+    lhs.free()
