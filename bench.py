@@ -528,13 +528,14 @@ def run_gsls(args):
     if roof64["achieved"] and not is_fluid(p):
         avg_s = roof64["avg_launch_us"] / 1e6
         t_fma, t_hbm = fmas / rate.value, roof64["bytes_per_launch"] / (peak * 1e9)
-        hbm = {k: roof64[k] for k in ("achieved", "peak", "unit", "frac", "peak_source", "traffic")}
+        mem = {k: roof64[k] for k in ("achieved", "peak", "unit", "frac", "peak_source", "traffic")}
+        mem_name = roof64["bound"]
         if t_fma > t_hbm:
             roof64.update({"bound": "fp64", "achieved": 2 * fmas / avg_s / 1e12,
                            "peak": 2 * rate.value / 1e12, "unit": "TFLOP/s",
                            "frac": t_fma / avg_s,
                            "peak_source": "measured FP64 FMA rate (gsls_fp64_fma_rate)",
-                           "fma_per_launch": fmas, "hbm": hbm})
+                           "fma_per_launch": fmas, mem_name: mem})
 
     out = {
         "metric": METRIC, "value": job_value(ms_mixed / 1e3, world), "unit": "s/step",

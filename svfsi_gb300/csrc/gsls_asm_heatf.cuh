@@ -41,9 +41,9 @@ __global__ void __launch_bounds__(kAsmThreads) k_asm_heatf(AsmArgs A) {
   // Nx_a^T.  The element runs on the FP64 pipe, so its quadratic forms are
   // taken through those gradients, x.ks.x = sum_{a<3} (Nx_a.x)^2 (u.ks.u
   // and Tx.ks.Tx), ks:ks comes from the geometry table, and what is linear in
-  // Nx_a is minus the sum of the other three at the fourth node: the
+  // Nx_a is minus the sum of the other three at the fourth node (in FP64): the
   // reference's quantities, rounded differently.  (Cylinder of 1,225,440
-  // tets, mixed, ten assemblies and solves: 13.6 ms before, 10.9 ms with the
+  // tets, mixed, ten assemblies and solves: 13.5 ms before, 11.1 ms with the
   // last two and the element buffer.)
   double kS, trk;
   load_metric(A, e, kS, trk);

@@ -62,7 +62,7 @@ __device__ __forceinline__ double jm23(double J) {
 // error of the largest, and a flat element's smallest gradient is a small part
 // of it.  sum_b M_ab x_b is m0 sum_b x_b + (m1 - m0) x_a.
 // Beam of 2,044,416 tets (FP32 tangent): 3.87 ms with the stress formed and
-// colour scatter, 2.94 ms in this form with colour scatter, 1.67 ms through
+// colour scatter, 2.94 ms in this form with colour scatter, 1.68 ms through
 // the element buffer.
 template <class VT>
 __global__ void __launch_bounds__(kAsmThreads, sizeof(VT) == 4 ? 4 : 3)

@@ -16,11 +16,11 @@
 // share, L1) still holds of the matrix is met first.
 //
 // Measured (GB300): the FP32 solves of the neo-Hookean beam (358,425 nodes,
-// 3x3 blocks, 208 MB of matrix) take ~41 us per iteration against 74 us for
-// the three batched kernels (an iteration reads 145 MB from DRAM, 21 us at
+// 3x3 blocks, 188 MB of matrix) take 36 us per iteration against 74 us for
+// the three batched kernels (an iteration reads 134 MB from DRAM, 20 us at
 // the measured copy rate; the rest is L2 and two grid sums of ~3.5 us); the
 // FP64 3x3 solves of 15,616 nodes 13 us against 21 us (FP64 pipe 5 us); the
-// 20^3 heat cube 7 us against 12 us per iteration (two grid sums).
+// 20^3 heat cube 8 us against 12 us per iteration (two grid sums).
 //
 // Staging the stream in shared memory by bulk copies (a ring per warp with an
 // mbarrier per slot, or one ring per block with a producer warp) was slower:
