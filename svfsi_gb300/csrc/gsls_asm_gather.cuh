@@ -201,6 +201,11 @@ __global__ void __launch_bounds__(256) k_gather_val(size_t n, const int *__restr
     for (int q = 0; q < V; q++) out[q] = s[q];
   }
 }
+// Residual values of an element in the buffer: 4 per degree of freedom; a scalar
+// element's are not weighted yet, its weight is the fifth of 6
+template <int DOF>
+constexpr int kResRow = DOF == 1 ? 6 : 4 * DOF;
+
 // R of a node from the list of its diagonal block, whose entries are (e, a, a)
 template <int DOF>
 __global__ void __launch_bounds__(256) k_gather_res(int nNo, const int *__restrict__ diagPtr,
@@ -217,20 +222,22 @@ __global__ void __launch_bounds__(256) k_gather_res(int nNo, const int *__restri
     double s = first ? 0.0 : R[k];
     for (int q = b; q < e; q += 4) {
       int id[4];
-      double v[4];
+      double v[4], w[4] = {};
 #pragma unroll
       for (int u = 0; u < 4; u++) {
         id[u] = q + u < e ? __ldg(ent + q + u) : -1;
         if (id[u] >= 0 && ((id[u] >> 4) < e0 || (id[u] >> 4) >= e1)) id[u] = -1;
       }
 #pragma unroll
-      for (int u = 0; u < 4; u++)
-        v[u] = id[u] >= 0
-                   ? __ldcs(lR + ((size_t)((id[u] >> 4) - e0) * 4 + (id[u] & 3)) * DOF + c)
-                   : 0.0;
+      for (int u = 0; u < 4; u++) {
+        const double *__restrict__ r =
+            lR + (size_t)((id[u] >= 0 ? id[u] >> 4 : e0) - e0) * kResRow<DOF>;
+        v[u] = id[u] >= 0 ? __ldcs(r + (id[u] & 3) * DOF + c) : 0.0;
+        if constexpr (DOF == 1) w[u] = id[u] >= 0 ? __ldcs(r + 4) : 0.0;
+      }
 #pragma unroll
       for (int u = 0; u < 4; u++)
-        if (id[u] >= 0) s += v[u];
+        if (id[u] >= 0) s = DOF == 1 ? fma(w[u], v[u], s) : s + v[u];
     }
     R[k] = s;
   }

@@ -40,21 +40,25 @@ __global__ void __launch_bounds__(kAsmThreads) k_asm_heatf(AsmArgs A) {
   // gradients of the first three shape functions, so ks = sum_{a<3} Nx_a
   // Nx_a^T.  The element runs on the FP64 pipe, so its quadratic forms are
   // taken through those gradients, x.ks.x = sum_{a<3} (Nx_a.x)^2 (u.ks.u
-  // and Tx.ks.Tx), ks:ks comes from the geometry table, and what is linear in
-  // Nx_a is minus the sum of the other three at the fourth node (in FP64): the
-  // reference's quantities, rounded differently.  (Cylinder of 1,225,440
-  // tets, mixed, ten assemblies and solves: 13.5 ms before, 11.1 ms with the
-  // last two and the element buffer.)
+  // and Tx.ks.Tx), and ks:ks comes from the geometry table: the reference's
+  // quantities, rounded differently.  (Cylinder of 1,225,440 tets, mixed, ten
+  // assemblies and solves: 13.5 ms before, 11.2 ms with the table and the
+  // element buffer.)
+  //
+  // The arithmetic keeps one order.  The diffusivity divides by |Tx|: where
+  // that nearly vanishes, one rounding moves a step that ends at its iteration
+  // limit by up to 1e-7 at a node, in every later step too.  Taking Tx from
+  // differences of nodal values, or what is linear in Nx_a as minus the other
+  // three's sum, saves 3 % of the FP64 work and is not done.
   double kS, trk;
   load_metric(A, e, kS, trk);
   double Tx[3];
 #pragma unroll
   for (int i = 0; i < 3; i++)
-    Tx[i] = Nx[i][0] * (Ty[0] - Ty[3]) + Nx[i][1] * (Ty[1] - Ty[3]) + Nx[i][2] * (Ty[2] - Ty[3]);
+    Tx[i] = Nx[i][0] * Ty[0] + Nx[i][1] * Ty[1] + Nx[i][2] * Ty[2] + Nx[i][3] * Ty[3];
   double NxTx[4];  // Nx_a . Tx (constant on a tet4)
 #pragma unroll
-  for (int a = 0; a < 3; a++) NxTx[a] = Nx[0][a] * Tx[0] + Nx[1][a] * Tx[1] + Nx[2][a] * Tx[2];
-  NxTx[3] = -(NxTx[0] + NxTx[1] + NxTx[2]);
+  for (int a = 0; a < 4; a++) NxTx[a] = Nx[0][a] * Tx[0] + Nx[1][a] * Tx[1] + Nx[2][a] * Tx[2];
   double nTx = NxTx[0] * NxTx[0] + NxTx[1] * NxTx[1] + NxTx[2] * NxTx[2];  // Tx.ks.Tx
   // ISZERO (MATFUN.f:763-780): |x| < eps^2
   if (fabs(nTx) < 4.930380657631324e-32) nTx = 2.220446049250313e-16;
@@ -99,9 +103,9 @@ __global__ void __launch_bounds__(kAsmThreads) k_asm_heatf(AsmArgs A) {
 #pragma unroll
     for (int i = 0; i < 3; i++) u[i] = ys[i] + rd * y[g][i];
     const double Td = Tas + rd * Ta[g];
-    double udNx[3];  // u . Nx_a
+    double udNx[4];  // u . Nx_a
 #pragma unroll
-    for (int a = 0; a < 3; a++) udNx[a] = u[0] * Nx[0][a] + u[1] * Nx[1][a] + u[2] * Nx[2][a];
+    for (int a = 0; a < 4; a++) udNx[a] = u[0] * Nx[0][a] + u[1] * Nx[1][a] + u[2] * Nx[2][a];
     const double kU = udNx[0] * udNx[0] + udNx[1] * udNx[1] + udNx[2] * udNx[2];  // u.ks.u
     const double udTx = u[0] * Tx[0] + u[1] * Tx[1] + u[2] * Tx[2];
     const double r = Td + udTx;
@@ -112,20 +116,16 @@ __global__ void __launch_bounds__(kAsmThreads) k_asm_heatf(AsmArgs A) {
     rsum += r;
     nusum += nu;
 #pragma unroll
-    for (int a = 0; a < 3; a++) lRu[a] += udNx[a] * tr;
-    // FP32 tangents: the fourth node's u.Nx is formed in FP64 and rounded as the
-    // others are (minus the sum of three rounded values has their error, which
-    // on a flat element is many times a small gradient), and the diffusive
-    // part is added point by point, in the order of the FP32 sum
+    for (int a = 0; a < 4; a++) lRu[a] += udNx[a] * tr;
+    // FP32 tangents: u.Nx of every node is rounded from FP64 (minus the sum of
+    // three rounded values has their error, which on a flat element is many
+    // times a small gradient), and the diffusive part is added point by point;
+    // in FP64 it is added once, which saves 48 of ~350 instructions
     const VT tv = VT(tauM), wn = VT(wl * nu);
-    VT ta[4], tb[4], uv[4];
-#pragma unroll
-    for (int a = 0; a < 3; a++) uv[a] = VT(udNx[a]);
-    uv[3] = f32 ? VT(u[0] * Nx[0][3] + u[1] * Nx[1][3] + u[2] * Nx[2][3])
-                : -(uv[0] + uv[1] + uv[2]);
+    VT ta[4], tb[4];
 #pragma unroll
     for (int a = 0; a < 4; a++) {
-      const VT un = uv[a], na = a == g ? nsv : ntv;
+      const VT un = VT(udNx[a]), na = a == g ? nsv : ntv;
       ta[a] = wlv * (na + tv * un);
       tb[a] = na * amdv + un;
     }
@@ -145,14 +145,15 @@ __global__ void __launch_bounds__(kAsmThreads) k_asm_heatf(AsmArgs A) {
 #pragma unroll
       for (int b = 0; b < 4; b++) lK[a][b] += nuv * NxN[a][b];
   }
-  lRu[3] = -(lRu[0] + lRu[1] + lRu[2]);
   double lR[4];
 #pragma unroll
   for (int a = 0; a < 4; a++) lR[a] = rt * rsum + rd * rg[a] + NxTx[a] * nusum + lRu[a];
-  // the element's 16 values and 4 residuals are whole vectors of their own
-  double2 *oR = reinterpret_cast<double2 *>(A.lR + (size_t)t * 4);
-  oR[0] = make_double2(w * lR[0], w * lR[1]);
-  oR[1] = make_double2(w * lR[2], w * lR[3]);
+  // the element's 16 values, and its 4 residuals with their weight, which
+  // k_gather_res applies, are whole vectors of their own
+  double2 *oR = reinterpret_cast<double2 *>(A.lR + (size_t)t * kResRow<1>);
+  oR[0] = make_double2(lR[0], lR[1]);
+  oR[1] = make_double2(lR[2], lR[3]);
+  oR[2] = make_double2(w, 0.0);
   uint4 *oK = reinterpret_cast<uint4 *>(reinterpret_cast<VT *>(A.lK) + (size_t)t * 16);
 #pragma unroll
   for (int q = 0; q < (int)sizeof(VT); q++) oK[q] = reinterpret_cast<const uint4 *>(&lK[0][0])[q];

@@ -199,17 +199,19 @@ __global__ void k_geo_tet4(int nEl, const int4 *__restrict__ ien, const double *
     N[i][2] = n2;
   }
   geo[(size_t)12 * nEl + e] = Jac;
-  double kk = 0.0, trk = 0.0;
+  double k00 = 0, k01 = 0, k02 = 0, k11 = 0, k12 = 0, k22 = 0;
 #pragma unroll
-  for (int i = 0; i < 3; i++)
-#pragma unroll
-    for (int j = i; j < 3; j++) {
-      const double k = N[i][0] * N[j][0] + N[i][1] * N[j][1] + N[i][2] * N[j][2];
-      kk += (i == j ? 1.0 : 2.0) * (k * k);
-      if (i == j) trk += k;
-    }
-  geo[(size_t)13 * nEl + e] = kk;
-  geo[(size_t)14 * nEl + e] = trk;
+  for (int a = 0; a < 3; a++) {
+    k00 += N[0][a] * N[0][a];
+    k01 += N[0][a] * N[1][a];
+    k02 += N[0][a] * N[2][a];
+    k11 += N[1][a] * N[1][a];
+    k12 += N[1][a] * N[2][a];
+    k22 += N[2][a] * N[2][a];
+  }
+  geo[(size_t)13 * nEl + e] =
+      k00 * k00 + k11 * k11 + k22 * k22 + 2.0 * (k01 * k01 + k02 * k02 + k12 * k12);
+  geo[(size_t)14 * nEl + e] = k00 + k11 + k22;
 }
 
 // ---------------------------------------------------------------------------
@@ -545,11 +547,11 @@ static int assemble_gather(gsls_mesh *m, K kern, size_t smem, AsmArgs A, double 
   constexpr int DD = DOF * DOF;
   gsls_lhs *lhs = m->lhs;
   cudaStream_t st = lhs->stream;
-  // matrices, then residuals (4 * DOF doubles: whole 16-byte vectors).  At most
+  // matrices, then residuals (whole 16-byte vectors).  At most
   // a quarter of the free memory, since a solver's workspaces are taken later;
   // smaller parts still where that cannot be had.  The size that was had is
   // kept: asking for more again would free the buffer each time.
-  constexpr size_t kEl = 16 * DD * sizeof(VT), kRes = 4 * DOF * sizeof(double);
+  constexpr size_t kEl = 16 * DD * sizeof(VT), kRes = kResRow<DOF> * sizeof(double);
   constexpr size_t per = kEl + kRes;
   static_assert(kEl % 16 == 0 && kRes % 16 == 0, "whole vectors");
   if (m->el_most == 0)
