@@ -88,10 +88,11 @@ typedef struct gsls_eq gsls_eq;     /* one equation's time integrator */
    fixed scratch array on it). */
 int gsls_init(int device);
 /* No counterpart in the reference.  Poll limit of the grid barrier that
-   the one-launch CG and Schur-complement CG wait on between their phases (0 = the default, 2^24 polls: seconds).  When a wait reaches the
-   limit the kernel sets an error word, every block leaves, and the solve
-   returns GSLS_ERR_CUDA with the CUDA context intact.  A test hook for the
-   timeout path; a small limit makes waits expire on healthy launches. */
+   the one-launch CG and Schur-complement CG wait on between their phases
+   (0 = the default, 2^24 polls: seconds).  When a wait reaches the limit the
+   kernel sets an error word, every block leaves, and the solve returns
+   GSLS_ERR_CUDA with the CUDA context intact.  A test hook for the timeout
+   path; a small limit makes waits expire on healthy launches. */
 int gsls_set_wait_limit(unsigned polls);
 /* No counterpart in the reference.  Device memory that the library may still
    take for the calling thread: a request above it fails as on a device that
